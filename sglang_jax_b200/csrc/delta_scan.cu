@@ -23,10 +23,20 @@
 namespace sglb {
 namespace {
 
+// Columns of a projection's row.  Heads that share a q / k head are neighbours and form a group; the q and k channels of group g
+// begin at column `q + g * qk_step` and `k + g * qk_step`, its value heads' channels at `v + g * v_step`, the inputs of its heads'
+// beta and decay at `b + g * ba_step` and `a + g * ba_step`.  One run of q, then k, then v channels: steps of one head (of one
+// group's value heads); the checkpoints that keep a group's q, k, v and gate rows together: steps of a whole group.
+struct DeltaColumns {
+  int q, k, qk_step, v, v_step, b, a, ba_step;
+};
+
 struct DeltaParams {
-  const void* proj;              // [T, ld]: q | k | v channels at column 0, gate / b / a at the offsets below
+  const void* proj;              // [T, ld]: the q, k and v channels, where `cols` says
   long long ld;
-  int g_off, b_off, a_off;
+  const void* ba;                // [T, ba_ld]: inputs of beta and decay, where `cols` says
+  long long ba_ld;
+  DeltaColumns cols;
   const void* conv_w;            // [channels, taps], channels = q | k | v
   const float* a_log;            // [H]
   const float* dt_bias;          // [H]; per channel: [H, D]
@@ -64,9 +74,10 @@ struct Conv {
         w[i][j] = (tap >= 0 && c < width) ? to_f(kernel[static_cast<long long>(c0 + c) * taps + tap]) : 0.f;
       }
   }
-  // window in front of row `start + local` of a sequence whose rows begin at `start`
+  // window in front of row `start + local` of a sequence whose rows begin at `start`; the channels from c0 on are the columns
+  // from `col` on
   __device__ __forceinline__ void load_window(const T* __restrict__ proj, long long ld, const T* __restrict__ stored,
-                                              bool fresh, int start, int local, int c0, int width, int taps, int lane) {
+                                              bool fresh, int start, int local, int col, int c0, int width, int taps, int lane) {
     const int win = taps - 1;
 #pragma unroll
     for (int i = 0; i < NPL; ++i)
@@ -75,7 +86,7 @@ struct Conv {
         const int c = lane + 32 * i, back = TAPS - 1 - j, r = local - back;
         float v = 0.f;
         if (c < width && back <= win) {
-          if (r >= 0) v = to_f(proj[(start + r) * ld + c0 + c]);
+          if (r >= 0) v = to_f(proj[(start + r) * ld + col + c]);
           else if (!fresh) v = to_f(stored[static_cast<long long>(c0 + c) * win + win + r]);
         }
         x[i][j] = v;
@@ -137,26 +148,27 @@ __global__ void __launch_bounds__(128) delta_prep_kernel(const DeltaParams p) {
     for (int i = 0; i < NPL; ++i) in[i] = lane + 32 * i < width ? to_f(src[lane + 32 * i]) : 0.f;
   };
   if (unit < p.Hk) {
-    const int q0 = unit * p.D, k0 = p.Hk * p.D + unit * p.D;
+    const int q0 = unit * p.D, k0 = p.Hk * p.D + unit * p.D;             // channels, and the columns they are found in
+    const int qc = p.cols.q + unit * p.cols.qk_step, kc = p.cols.k + unit * p.cols.qk_step;
     Conv<T, NPL, TAPS> cq, ck;
     cq.load_kernel(kernel, q0, p.D, taps, lane);
     ck.load_kernel(kernel, k0, p.D, taps, lane);
     const float scale = 1.f / sqrtf(static_cast<float>(p.D));
     float in_q[NPL], in_k[NPL];
-    rows(t0, q0, p.D, in_q);
-    rows(t0, k0, p.D, in_k);
+    rows(t0, qc, p.D, in_q);
+    rows(t0, kc, p.D, in_k);
     walk(
         [&](const T* stored, bool fresh, int start, int local) {
-          cq.load_window(proj, p.ld, stored, fresh, start, local, q0, p.D, taps, lane);
-          ck.load_window(proj, p.ld, stored, fresh, start, local, k0, p.D, taps, lane);
+          cq.load_window(proj, p.ld, stored, fresh, start, local, qc, q0, p.D, taps, lane);
+          ck.load_window(proj, p.ld, stored, fresh, start, local, kc, k0, p.D, taps, lane);
         },
         [&](int t) {
           float q[NPL], k[NPL];
           cq.step(in_q, q);
           ck.step(in_k, k);
           if (t + 1 < t1) {                            // the next row is on its way while this one is worked on
-            rows(t + 1, q0, p.D, in_q);
-            rows(t + 1, k0, p.D, in_k);
+            rows(t + 1, qc, p.D, in_q);
+            rows(t + 1, kc, p.D, in_k);
           }
           float qq = 0.f, kk = 0.f;
 #pragma unroll
@@ -181,21 +193,22 @@ __global__ void __launch_bounds__(128) delta_prep_kernel(const DeltaParams p) {
           }
         });
   } else {
-    const int h = unit - p.Hk;
+    const int h = unit - p.Hk, r = p.H / p.Hk, hk = h / r;
     for (int vb = 0; vb < p.V; vb += 32 * NPL) {
       const int v0 = 2 * p.Hk * p.D + h * p.V + vb, width = min(32 * NPL, p.V - vb);
+      const int vc = p.cols.v + hk * p.cols.v_step + (h - hk * r) * p.V + vb;
       Conv<T, NPL, TAPS> cv;
       cv.load_kernel(kernel, v0, width, taps, lane);
       float in[NPL];
-      rows(t0, v0, width, in);
+      rows(t0, vc, width, in);
       walk(
           [&](const T* stored, bool fresh, int start, int local) {
-            cv.load_window(proj, p.ld, stored, fresh, start, local, v0, width, taps, lane);
+            cv.load_window(proj, p.ld, stored, fresh, start, local, vc, v0, width, taps, lane);
           },
           [&](int t) {
             float v[NPL];
             cv.step(in, v);
-            if (t + 1 < t1) rows(t + 1, v0, width, in);
+            if (t + 1 < t1) rows(t + 1, vc, width, in);
             float* dst = p.v + (static_cast<long long>(t) * p.H + h) * p.V + vb;
 #pragma unroll
             for (int i = 0; i < NPL; ++i)
@@ -203,10 +216,10 @@ __global__ void __launch_bounds__(128) delta_prep_kernel(const DeltaParams p) {
           });
     }
     for (int t = t0 + lane; t < t1; t += 32) {
-      const T* row = proj + static_cast<long long>(t) * p.ld;
+      const T* row = static_cast<const T*>(p.ba) + static_cast<long long>(t) * p.ba_ld + hk * p.cols.ba_step + (h - hk * r);
       float* gb = p.gb + (static_cast<long long>(t) * p.H + h) * 2;
-      if (p.chan_a == nullptr) gb[0] = expf(-expf(p.a_log[h]) * softplus(to_f(row[p.a_off + h]) + p.dt_bias[h]));
-      gb[1] = 1.f / (1.f + expf(-to_f(row[p.b_off + h])));
+      if (p.chan_a == nullptr) gb[0] = expf(-expf(p.a_log[h]) * softplus(to_f(row[p.cols.a]) + p.dt_bias[h]));
+      gb[1] = 1.f / (1.f + expf(-to_f(row[p.cols.b])));
     }
   }
 }
@@ -573,15 +586,17 @@ __device__ __forceinline__ void write_windows(const DeltaParams& p, int b, int h
   const T* proj = static_cast<const T*>(p.proj) + start * p.ld;
   T* cs = static_cast<T*>(p.conv_state);
   T* own = cs + p.slots[b] * channels * win;
-  auto window = [&](int c) {
+  auto window = [&](int c, int col) {
     T* keep = track > 0 && track <= n ? cs + (static_cast<long long>(p.track_slot[b]) * channels + c) * win : nullptr;
-    advance_window(own + static_cast<long long>(c) * win, keep, proj + c, p.ld, win, n, fresh, track);
+    advance_window(own + static_cast<long long>(c) * win, keep, proj + col, p.ld, win, n, fresh, track);
   };
-  for (int i = threadIdx.x; i < V; i += threads) window(2 * p.Hk * D + h * V + i);
-  if (h % (p.H / p.Hk) == 0)
+  const int first = h - hk * (p.H / p.Hk);             // place of the head in its group
+  for (int i = threadIdx.x; i < V; i += threads)
+    window(2 * p.Hk * D + h * V + i, p.cols.v + hk * p.cols.v_step + first * V + i);
+  if (first == 0)
     for (int i = threadIdx.x; i < D; i += threads) {
-      window(hk * D + i);
-      window(p.Hk * D + hk * D + i);
+      window(hk * D + i, p.cols.q + hk * p.cols.qk_step + i);
+      window(p.Hk * D + hk * D + i, p.cols.k + hk * p.cols.qk_step + i);
     }
 }
 
@@ -939,9 +954,22 @@ __global__ void __launch_bounds__(kStepThreads) delta_step_kernel(const DeltaPar
 
 // One warp per (token, head); a lane holds NV groups of four adjacent columns (V <= 128 * NV, V % 4 == 0), or takes single
 // columns (NV = 0, any V).
-template <typename T, int NV, bool SIGMOID>
-__global__ void delta_gate_kernel(const float* __restrict__ o, const T* __restrict__ gate, long long ld,
-                                  const float* __restrict__ w, T* __restrict__ out, long long T_, int H, int V, float eps) {
+// The gates of head h lie at column (h / group) * step + (h % group) * V of a row.
+template <typename W>
+__device__ __forceinline__ float4 load_weight4(const W* w) {
+  if constexpr (sizeof(W) == 2) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(w);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+  } else {
+    return *reinterpret_cast<const float4*>(w);
+  }
+}
+
+template <typename T, typename W, int NV, bool SIGMOID>
+__global__ void delta_gate_kernel(const float* __restrict__ o, const T* __restrict__ gate, long long ld, int group, int step,
+                                  const W* __restrict__ w, T* __restrict__ out, long long T_, int H, int V, float eps) {
   pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long wid = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
@@ -949,7 +977,7 @@ __global__ void delta_gate_kernel(const float* __restrict__ o, const T* __restri
   const long long t = wid / H;
   const int h = static_cast<int>(wid - t * H);
   const float* src = o + wid * V;
-  const T* g = gate + t * ld + static_cast<long long>(h) * V;
+  const T* g = gate + t * ld + static_cast<long long>(h / group) * step + static_cast<long long>(h % group) * V;
   T* dst = out + wid * V;
   auto gated = [](float x, float gv) { return x * ((SIGMOID ? 1.f : gv) / (1.f + expf(-gv))); };
   float ss = 0.f;
@@ -966,7 +994,7 @@ __global__ void delta_gate_kernel(const float* __restrict__ o, const T* __restri
     for (int i = 0; i < NV; ++i) {
       const int c = (lane + 32 * i) * 4;
       if (c >= V) continue;
-      const float4 wv = *reinterpret_cast<const float4*>(w + c);
+      const float4 wv = load_weight4(w + c);
       if constexpr (sizeof(T) == 2) {
         const uint2 raw = *reinterpret_cast<const uint2*>(g + c);
         const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
@@ -984,21 +1012,32 @@ __global__ void delta_gate_kernel(const float* __restrict__ o, const T* __restri
   } else {
     for (int i = lane; i < V; i += 32) ss += src[i] * src[i];
     const float inv = 1.f / sqrtf(warp_sum(ss) / V + eps);
-    for (int i = lane; i < V; i += 32) dst[i] = from_f<T>(gated(src[i] * inv * w[i], to_f(g[i])));
+    for (int i = lane; i < V; i += 32) dst[i] = from_f<T>(gated(src[i] * inv * to_f(w[i]), to_f(g[i])));
   }
 }
 
-template <typename T, bool SIGMOID>
-int run_gate(const float* o, const void* gate, long long ld, const float* w, void* out, long long n, int H, int V,
-             float eps, cudaStream_t s) {
+template <typename T, typename W, bool SIGMOID>
+int run_gate(const float* o, const void* gate, long long ld, int group, int step, const W* w, void* out, long long n, int H,
+             int V, float eps, cudaStream_t s) {
   const dim3 grid(static_cast<unsigned>((n * H + 3) / 4));
   const T* g = static_cast<const T*>(gate);
   T* d = static_cast<T*>(out);
-  const bool vec = V % 4 == 0 && ld % 4 == 0 && reinterpret_cast<uintptr_t>(gate) % (4 * sizeof(T)) == 0;
-  if (vec && V <= 128) launch_pdl(delta_gate_kernel<T, 1, SIGMOID>, grid, dim3(128), 0, s, o, g, ld, w, d, n, H, V, eps);
-  else if (vec && V <= 256) launch_pdl(delta_gate_kernel<T, 2, SIGMOID>, grid, dim3(128), 0, s, o, g, ld, w, d, n, H, V, eps);
-  else launch_pdl(delta_gate_kernel<T, 0, SIGMOID>, grid, dim3(128), 0, s, o, g, ld, w, d, n, H, V, eps);
+  const bool vec = V % 4 == 0 && ld % 4 == 0 && step % 4 == 0 && reinterpret_cast<uintptr_t>(gate) % (4 * sizeof(T)) == 0 &&
+                   reinterpret_cast<uintptr_t>(w) % (4 * sizeof(W)) == 0;
+  if (vec && V <= 128)
+    launch_pdl(delta_gate_kernel<T, W, 1, SIGMOID>, grid, dim3(128), 0, s, o, g, ld, group, step, w, d, n, H, V, eps);
+  else if (vec && V <= 256)
+    launch_pdl(delta_gate_kernel<T, W, 2, SIGMOID>, grid, dim3(128), 0, s, o, g, ld, group, step, w, d, n, H, V, eps);
+  else
+    launch_pdl(delta_gate_kernel<T, W, 0, SIGMOID>, grid, dim3(128), 0, s, o, g, ld, group, step, w, d, n, H, V, eps);
   return static_cast<int>(cudaGetLastError());
+}
+
+template <typename T, bool SIGMOID>
+int run_gate(const float* o, const void* gate, long long ld, int group, int step, const void* w, int w_f32, void* out,
+             long long n, int H, int V, float eps, cudaStream_t s) {
+  if (w_f32) return run_gate<T, float, SIGMOID>(o, gate, ld, group, step, static_cast<const float*>(w), out, n, H, V, eps, s);
+  return run_gate<T, __nv_bfloat16, SIGMOID>(o, gate, ld, group, step, static_cast<const __nv_bfloat16*>(w), out, n, H, V, eps, s);
 }
 
 template <typename T, int NPL, int TAPS>
@@ -1090,8 +1129,9 @@ int run_delta(const DeltaParams& p, cudaStream_t s) {
 
 extern "C" {
 
-// Shapes in DeltaParams; T = bf16 or fp32 (`is_f32`) is the type of `proj`, `conv_w` and `conv_state`.
-int sglb_delta_scan(const void* proj, long long ld, int g_off, int b_off, int a_off, const void* conv_w,
+// Shapes in DeltaParams, `cols` the eight members of DeltaColumns; T = bf16 or fp32 (`is_f32`) is the type of `proj`, `ba`,
+// `conv_w` and `conv_state`.
+int sglb_delta_scan(const void* proj, long long ld, const void* ba, long long ba_ld, const int* cols, const void* conv_w,
                     const float* a_log, const float* dt_bias, const void* chan_a, void* conv_state, float* state,
                     const long long* slots, const int* cu, const int* prefix, const int* track_len, const int* track_slot,
                     float* qk, float* v, float* gb, float* coef, float* kq, float* gc, float* o, int B, int T, int H, int Hk,
@@ -1101,21 +1141,24 @@ int sglb_delta_scan(const void* proj, long long ld, int g_off, int b_off, int a_
   if (cu != nullptr && (prefix == nullptr || (coef == nullptr && singles != B))) return -kBadArgument;
   if (chan_a != nullptr && coef != nullptr && (kq == nullptr || gc == nullptr)) return -kBadArgument;
   if (D < 1 || D > 256 || V < 1 || Hk < 1 || H % Hk != 0 || taps < 1 || taps > 16 || H > 65535) return -kBadArgument;
-  DeltaParams p{proj, ld, g_off, b_off, a_off, conv_w, a_log, dt_bias, chan_a, conv_state, state, slots, cu, prefix,
+  const DeltaColumns c{cols[0], cols[1], cols[2], cols[3], cols[4], cols[5], cols[6], cols[7]};
+  DeltaParams p{proj, ld, ba, ba_ld, c, conv_w, a_log, dt_bias, chan_a, conv_state, state, slots, cu, prefix,
                 track_len, track_slot, qk, v, gb, coef, kq, gc, o, B, T, H, Hk, D, V, taps, singles};
   return is_f32 ? run_delta<float>(p, s) : run_delta<__nv_bfloat16>(p, s);
 }
 
-// out [T, H * V] = rmsnorm(o [T, H, V], over V) * w [V] * silu(gate) (or sigmoid(gate)), gate at row stride `ld`.
-int sglb_delta_gate(const float* o, const void* gate, long long ld, const float* w, void* out, long long T, int H, int V,
-                    float eps, int sigmoid, int is_f32, cudaStream_t s) {
+// out [T, H * V] = rmsnorm(o [T, H, V], over V) * w [V] * silu(gate) (or sigmoid(gate)), gate at row stride `ld`, its heads in
+// groups of `group` neighbours `step` columns apart.
+int sglb_delta_gate(const float* o, const void* gate, long long ld, int group, int step, const void* w, int w_f32, void* out,
+                    long long T, int H, int V, float eps, int sigmoid, int is_f32, cudaStream_t s) {
   using namespace sglb;
   if (T <= 0) return 0;
+  if (group < 1) return -kBadArgument;
   if (sigmoid)
-    return is_f32 ? run_gate<float, true>(o, gate, ld, w, out, T, H, V, eps, s)
-                  : run_gate<__nv_bfloat16, true>(o, gate, ld, w, out, T, H, V, eps, s);
-  return is_f32 ? run_gate<float, false>(o, gate, ld, w, out, T, H, V, eps, s)
-                : run_gate<__nv_bfloat16, false>(o, gate, ld, w, out, T, H, V, eps, s);
+    return is_f32 ? run_gate<float, true>(o, gate, ld, group, step, w, w_f32, out, T, H, V, eps, s)
+                  : run_gate<__nv_bfloat16, true>(o, gate, ld, group, step, w, w_f32, out, T, H, V, eps, s);
+  return is_f32 ? run_gate<float, false>(o, gate, ld, group, step, w, w_f32, out, T, H, V, eps, s)
+                : run_gate<__nv_bfloat16, false>(o, gate, ld, group, step, w, w_f32, out, T, H, V, eps, s);
 }
 
 }  // extern "C"

@@ -1039,7 +1039,7 @@ int sglb_gemm_bf16_impl(const void* x, const void* w, const void* bias, void* ou
                         void* workspace, size_t workspace_bytes, int* counters, int force_mode, int force_splits,
                         void* const* rs_peers, int rs_world, int rs_rank, cudaStream_t stream,
                         const float* scale_x = nullptr, const float* scale_w = nullptr,
-                        const SglbFusedHost* fused = nullptr);
+                        const SglbFusedHost* fused = nullptr, long long ldx = 0);
 
 // out[M,N] (bf16) = (x_q[M,K] . w_q[N,K]^T) * scale_x[M] * scale_w[N] + bias with e4m3 operands
 // (per-token activation scales, per-output-channel weight scales; K a multiple of 16).
@@ -1055,6 +1055,13 @@ int sglb_gemm_bf16(const void* x, const void* w, const void* bias, void* out, in
                    size_t workspace_bytes, int* counters, int force_mode, int force_splits, cudaStream_t stream) {
   return sglb_gemm_bf16_impl(x, w, bias, out, M, N, K, workspace, workspace_bytes, counters, force_mode, force_splits,
                              nullptr, 0, 0, stream);
+}
+
+// The same for rows of x that are `ldx` elements apart (a multiple of 8: whole 16-byte units): a column range of a wider product.
+int sglb_gemm_bf16_ld(const void* x, long long ldx, const void* w, const void* bias, void* out, int M, int N, int K,
+                      void* workspace, size_t workspace_bytes, int* counters, cudaStream_t stream) {
+  return sglb_gemm_bf16_impl(x, w, bias, out, M, N, K, workspace, workspace_bytes, counters, -1, 0, nullptr, 0, 0, stream,
+                             nullptr, nullptr, nullptr, ldx);
 }
 
 // Row-parallel GEMM whose epilogue performs the reduce-scatter sends: `rs_peers[r]` is rank r's
@@ -1084,11 +1091,13 @@ void sglb_gemm_set_debug_stamps(void* dev_ptr) { g_debug_stamps = static_cast<un
 int sglb_gemm_bf16_impl(const void* x, const void* w, const void* bias, void* out, int M, int N, int K,
                         void* workspace, size_t workspace_bytes, int* counters, int force_mode, int force_splits,
                         void* const* rs_peers, int rs_world, int rs_rank, cudaStream_t stream,
-                        const float* scale_x, const float* scale_w, const SglbFusedHost* fused) {
+                        const float* scale_x, const float* scale_w, const SglbFusedHost* fused, long long ldx) {
   using namespace sglb;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((K % 8) || (N % 8)) return -kBadArgument;
   const bool fp8 = scale_x != nullptr;
+  if (ldx == 0) ldx = K;
+  if (ldx < K || (ldx * (fp8 ? 1 : 2)) % 16 != 0) return -kBadArgument;
   const int eb = fp8 ? 1 : 2;                          // operand element bytes
   const int bke = fp8 ? 2 * BK : BK;                   // elements per 128-byte K block
   const int kb_total = (K + bke - 1) / bke;
@@ -1162,7 +1171,7 @@ int sglb_gemm_bf16_impl(const void* x, const void* w, const void* bias, void* ou
                        ? 256 : 128;
     p.tiles_a = (M + BM - 1) / BM;
     p.tiles_b = (N + bn - 1) / bn;
-    if (!encode_tmap_2d(&ta, x, K, M, static_cast<uint64_t>(K) * eb, bke, BM, eb)) return -100;
+    if (!encode_tmap_2d(&ta, x, K, M, static_cast<uint64_t>(ldx) * eb, bke, BM, eb)) return -100;
     if (!encode_tmap_2d(&tb, w, K, N, static_cast<uint64_t>(K) * eb, bke, bn, eb)) return -101;
     int grid = min(p.tiles_a * p.tiles_b, sms);
     if (M <= 256 && force_splits <= 0 && workspace != nullptr && counters != nullptr) {
@@ -1218,7 +1227,7 @@ int sglb_gemm_bf16_impl(const void* x, const void* w, const void* bias, void* ou
     }
     p.splits = splits;
     if (!encode_tmap_2d(&ta, w, K, N, static_cast<uint64_t>(K) * eb, bke, BM, eb)) return -100;
-    if (!encode_tmap_2d(&tb, x, K, M, static_cast<uint64_t>(K) * eb, bke, bn, eb)) return -101;
+    if (!encode_tmap_2d(&tb, x, K, M, static_cast<uint64_t>(ldx) * eb, bke, bn, eb)) return -101;
     if (fp8) {
       switch (bn) {
         case 16: err = launch<16, 1, true>(ta, tb, p, grid, stream); break;

@@ -134,6 +134,48 @@ class PackedColumnParallelLinear(LinearBase):
         param.data.narrow(0, off, n).copy_(w.narrow(0, self.tp_rank // int(split) * n if split else 0, n))
 
 
+class JointProjection:
+    """Several projections of one input as a single product, while each stays a layer of its own: their weights are made
+    neighbours in one allocation, so that one product over all of them gives every result as a column range.  `joint(x)` is
+    None where that does not hold (any more): a layer with a bias, quantised or with an adapter, another type for one of them, a
+    weight that was replaced or moved.  Whether it does is read off the weights themselves on every call."""
+
+    def __init__(self, linears: list[LinearBase]):
+        self.linears = linears
+        w = [lin.weight for lin in linears]
+        # whole 16-byte units: every column range keeps the alignment of the rows
+        if all(t is not None and t.dtype == w[0].dtype and t.shape[1] == w[0].shape[1] and t.shape[0] % 8 == 0 for t in w):
+            base = torch.empty(sum(t.shape[0] for t in w), w[0].shape[1], dtype=w[0].dtype, device=w[0].device)
+            row = 0
+            for lin, t in zip(linears, w):
+                lin.weight = nn.Parameter(base.narrow(0, row, t.shape[0]), requires_grad=False)
+                row += t.shape[0]
+
+    def weight(self) -> torch.Tensor | None:
+        """The weights as one matrix, or None."""
+        first = self.linears[0].weight
+        if first is None:
+            return None
+        at, rows, K = first.data_ptr(), 0, first.shape[1]
+        for lin in self.linears:
+            w = lin.weight
+            if (w is None or lin.qweight is not None or lin.lora is not None or lin.bias is not None or w.dtype != first.dtype
+                    or w.data_ptr() != at or w.shape[1] != K or not w.is_contiguous()
+                    or w.untyped_storage().data_ptr() != first.untyped_storage().data_ptr()):
+                return None
+            at += w.numel() * w.element_size()
+            rows += w.shape[0]
+        return torch.as_strided(first, (rows, K), (K, 1))
+
+    def __call__(self, x: torch.Tensor) -> tuple[torch.Tensor, list[torch.Tensor]] | None:
+        """All products in one tensor, and each as a column range of it."""
+        w = self.weight()
+        if w is None:
+            return None
+        y = ops.linear(x, w)
+        return y, list(y.split([lin.weight.shape[0] for lin in self.linears], -1))
+
+
 class QKVParallelLinear(LinearBase):
     """Fused q/k/v projection.  Query heads are split over ranks; KV heads are split
     when `tp <= kv_heads` and replicated otherwise (reference

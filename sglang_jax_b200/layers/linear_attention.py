@@ -15,7 +15,7 @@ from .. import ops
 from ..ops import linear_attention as la
 from ..parallel import state as ps
 from .layernorm import GatedRMSNorm
-from .linear import PackedColumnParallelLinear, ReplicatedLinear, RowParallelLinear
+from .linear import JointProjection, PackedColumnParallelLinear, ReplicatedLinear, RowParallelLinear
 
 
 def track_pieces(a0: int, a1: int, track):
@@ -39,14 +39,6 @@ def recurrent_slots(fb) -> torch.Tensor:
     return slots if slots is not None else fb.req_pool_indices.long() + 1
 
 
-def _native_step_ok(x, conv_all, rec_all, dk: int, dv: int) -> bool:
-    """Whether a decode step can run the in-place CUDA kernels (`csrc/linear_attn.cu`)."""
-    from .. import ops
-    return (ops.use_native(x) and rec_all.dtype == torch.float32 and conv_all.dtype in (torch.bfloat16, torch.float32)
-            and rec_all.is_contiguous() and conv_all.is_contiguous() and dk <= 256 and dv <= 256 and dv % 32 == 0
-            and conv_all.shape[-1] + 1 <= 8)
-
-
 class GatedDeltaNet(nn.Module):
     def __init__(self, config, linear_layer_index: int, dtype):
         super().__init__()
@@ -66,6 +58,7 @@ class GatedDeltaNet(nn.Module):
         self.A_log = nn.Parameter(torch.zeros(self.nv, dtype=torch.float32), requires_grad=False)
         self.norm = GatedRMSNorm(self.dv, config.rms_norm_eps, dtype)
         self.out_proj = ReplicatedLinear(self.value_dim, H, False, dtype)
+        self._joint = JointProjection([self.in_proj_qkvz, self.in_proj_ba])
 
     def weight_loader(self, param, w, shard_id=None):
         if w.dim() == 3:                 # depth-wise conv kernel stored [C, 1, K]
@@ -86,6 +79,15 @@ class GatedDeltaNet(nn.Module):
         fb = forward_batch
         pool = fb.extras["recurrent_pool"]
         conv_all, rec_all = pool.conv_state[self.layer_index], pool.recurrent_state[self.layer_index]
+        if ops.delta_supported(x, conv_all, rec_all, self.dk, self.dv, self.conv_kernel) and self.conv1d_weight.dtype == x.dtype:
+            joint = self._joint(x)
+            qkvz, ba = joint[1] if joint is not None else (self.in_proj_qkvz(x), self.in_proj_ba(x))
+            r = self.nv // self.nk
+            group = 2 * self.dk + 2 * r * self.dv                      # q, k, values and gates of one key head
+            o = ops.delta_scan(qkvz, -1, 0, r, self.conv1d_weight, self.A_log.float(), self.dt_bias.float(), conv_all, rec_all,
+                               recurrent_slots(fb), self.nv, self.nk, self.dk, self.dv, ba=ba, grouped=group, **ragged_step(fb))
+            gate = qkvz[:, 2 * self.dk + r * self.dv:]
+            return self.out_proj(ops.delta_gate(o, gate, self.norm.weight, self.norm.eps, group=r, step=group))
         q, k, v, z, b, a = self._split(self.in_proj_qkvz(x), self.in_proj_ba(x))
         mixed = torch.cat([q, k, v], dim=-1)                             # [T, conv_dim]
         beta = torch.sigmoid(b.float())
@@ -102,14 +104,7 @@ class GatedDeltaNet(nn.Module):
                 qq, kk = qq.repeat_interleave(r, 1), kk.repeat_interleave(r, 1)
             return qq, kk, vv.reshape(-1, self.nv, self.dv)
 
-        if fb.forward_mode.is_decode() and _native_step_ok(x, conv_all, rec_all, self.dk, self.dv):
-            # sm_100a path: the convolution window and the state matrix are updated in place in their pools
-            from ..ops import native
-            y = native.conv1d_update(mixed, conv_all, self.conv1d_weight, slots)
-            qq, kk, vv = torch.split(y, [self.key_dim, self.key_dim, self.value_dim], dim=-1)
-            o = native.delta_rule_step(qq.reshape(T, self.nk, self.dk), kk.reshape(T, self.nk, self.dk),
-                                       vv.reshape(T, self.nv, self.dv), g, beta, rec_all, slots)
-        elif fb.forward_mode.is_decode():
+        if fb.forward_mode.is_decode():
             y, new_conv = la.causal_conv1d_update(mixed, conv_all[slots], self.conv1d_weight)
             conv_all[slots] = new_conv.to(conv_all.dtype)
             qq, kk, vv = heads(y)
@@ -355,15 +350,50 @@ class KimiDeltaAttention(_RecurrentMixer):
         self.o_norm = GatedRMSNorm(self.hd, config.rms_norm_eps, dtype)
         self.o_norm.gate_act = "sigmoid"
         self.o_proj = ReplicatedLinear(P, H, False, dtype)
+        self._joint = JointProjection([self.q_proj, self.k_proj, self.v_proj, self.f_a_proj, self.g_a_proj, self.b_proj])
+        # the three kernels of the convolution are neighbours, too (`_conv_weight`)
+        taps = torch.empty(3 * P, self.conv_kernel, dtype=dtype)
+        for i, name in enumerate(self._CONV):
+            setattr(self, name, nn.Parameter(taps.narrow(0, i * P, P), requires_grad=False))
+
+    _CONV = ("q_conv1d_weight", "k_conv1d_weight", "v_conv1d_weight")
+
+    def _conv_weight(self) -> torch.Tensor:
+        """Kernels of the q, k and v channels as one matrix, copied only if they are no longer neighbours."""
+        w = [getattr(self, name) for name in self._CONV]
+        step = w[0].numel() * w[0].element_size()
+        if all(t.is_contiguous() and t.dtype == w[0].dtype and t.data_ptr() == w[0].data_ptr() + i * step
+               and t.untyped_storage().data_ptr() == w[0].untyped_storage().data_ptr() for i, t in enumerate(w)):
+            return torch.as_strided(w[0], (3 * w[0].shape[0], w[0].shape[1]), (w[0].shape[1], 1))
+        return torch.cat(w, 0)
 
     def weight_loader(self, param, w, shard_id=None):
         param.data.copy_((w.squeeze(1) if w.dim() == 3 else w).reshape(param.shape).to(param.dtype))
 
+    @staticmethod
+    def _up(lin, part):
+        """Second product of a low-rank pair; a plain layer reads the column range of the wider product where it is."""
+        if lin.qweight is None and lin.lora is None and lin.bias is None and lin.weight.dtype == part.dtype:
+            return ops.linear_part(part, lin.weight)
+        return lin(part.contiguous())
+
     def forward(self, x, fb):
         T = x.shape[0]
         nh, hd = self.nh, self.hd
+        w = self._conv_weight()
+        pool = fb.extras["recurrent_pool"]
+        conv_all, rec_all = pool.conv_state[self.layer_index], pool.recurrent_state[self.layer_index]
+        if ops.delta_supported(x, conv_all, rec_all, hd, hd, self.conv_kernel) and w.dtype == x.dtype:
+            joint = self._joint(x)
+            if joint is not None:
+                qkv, f, g, ba = joint[0], joint[1][3], joint[1][4], joint[1][5]
+            else:
+                qkv = torch.cat([self.q_proj(x), self.k_proj(x), self.v_proj(x)], -1)
+                f, g, ba = self.f_a_proj(x), self.g_a_proj(x), self.b_proj(x)
+            o = ops.delta_scan(qkv, -1, 0, -1, w, self.A_log.float(), self.dt_bias.float(), conv_all, rec_all, recurrent_slots(fb),
+                               nh, nh, hd, hd, channel_a=self._up(self.f_b_proj, f), ba=ba, **ragged_step(fb))
+            return self.o_proj(ops.delta_gate(o, self._up(self.g_b_proj, g), self.o_norm.weight, self.o_norm.eps, "sigmoid"))
         mixed = torch.cat([self.q_proj(x), self.k_proj(x), self.v_proj(x)], -1)
-        w = torch.cat([self.q_conv1d_weight, self.k_conv1d_weight, self.v_conv1d_weight], 0)
         raw = self.f_b_proj(self.f_a_proj(x)).view(T, nh, hd).float() + self.dt_bias.view(nh, hd)
         g = -self.A_log.float().exp().view(1, nh, 1) * torch.nn.functional.softplus(raw)
         beta = torch.sigmoid(self.b_proj(x).float())
@@ -382,10 +412,6 @@ class KimiDeltaAttention(_RecurrentMixer):
             return o[0]
 
         def per_batch(conv_all, rec_all, slots):
-            if _native_step_ok(x, conv_all, rec_all, hd, hd):
-                from ..ops import native
-                q, k, v = split(native.conv1d_update(mixed, conv_all, w, slots))
-                return native.delta_rule_step(q, k, v, g, beta, rec_all, slots, gate_per_channel=True)
             y, cs = la.causal_conv1d_update(mixed, conv_all[slots], w)
             conv_all[slots] = cs.to(conv_all.dtype)
             q, k, v = split(y)

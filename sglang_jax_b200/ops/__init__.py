@@ -172,9 +172,22 @@ def delta_scan(proj, *a, **kw):
     return (_native() if use_native_wide(proj) else reference).delta_scan(proj, *a, **kw)
 
 
-def delta_gate(o, gate, weight, eps, act: str = "silu"):
-    """`rmsnorm(o) * weight * act(gate)` per head, act silu or sigmoid."""
-    return (_native() if use_native_wide(gate) else reference).delta_gate(o, gate, weight, eps, act)
+def delta_gate(o, gate, weight, eps, act: str = "silu", **kw):
+    """`rmsnorm(o) * weight * act(gate)` per head, act silu or sigmoid (`kw`: see `native.delta_gate`)."""
+    return (_native() if use_native_wide(gate) else reference).delta_gate(o, gate, weight, eps, act, **kw)
+
+
+def delta_supported(x, conv_state, state, dim: int, vdim: int, taps: int) -> bool:
+    """Whether `delta_scan` runs as kernels for these inputs and pools (the statements of `ops/linear_attention.py` otherwise)."""
+    return (use_native_wide(x) and conv_state.dtype == x.dtype and state.dtype == torch.float32 and conv_state.is_contiguous()
+            and state.is_contiguous() and 1 <= dim <= 256 and vdim >= 1 and 2 <= taps <= 16)
+
+
+def linear_part(x, w):
+    """`x @ w^T` of a column range of a wider product."""
+    if use_native(x) and w.dtype == torch.bfloat16:
+        return _native().linear_part(x, w)
+    return reference.linear(x, w)
 
 
 # ---- windowed attention over `PackedKVPool` rows (see `native.attn_prep`)

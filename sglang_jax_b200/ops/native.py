@@ -62,6 +62,8 @@ def lib():
     sig("sglb_gemm_max_counters", [c_int])
     sig("sglb_gemm_bf16", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_size_t,
                                  c_void_p, c_int, c_int, c_void_p])
+    sig("sglb_gemm_bf16_ld", [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_size_t,
+                              c_void_p, c_void_p])
     sig("sglb_rmsnorm", [c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_float, c_int, c_void_p])
     sig("sglb_fused_add_rmsnorm", [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_float, c_int,
                                          c_void_p])
@@ -121,9 +123,9 @@ def lib():
     sig("sglb_latent_extend_supported", [c_int, c_int, c_int])
     sig("sglb_latent_extend", [c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_int]
         + [c_void_p] * 5 + [c_int] * 6 + [c_float, c_int, c_void_p, c_void_p])
-    sig("sglb_delta_scan", [c_void_p, c_longlong, c_int, c_int, c_int] + [c_void_p] * 18 + [c_int] * 9 + [c_void_p])
-    sig("sglb_delta_gate", [c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_int, c_int, c_float, c_int,
-                            c_int, c_void_p])
+    sig("sglb_delta_scan", [c_void_p, c_longlong, c_void_p, c_longlong] + [c_void_p] * 19 + [c_int] * 9 + [c_void_p])
+    sig("sglb_delta_gate", [c_void_p, c_void_p, c_longlong, c_int, c_int, c_void_p, c_int, c_void_p, c_longlong, c_int, c_int,
+                            c_float, c_int, c_int, c_void_p])
     sig("sglb_attn_prep", [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_longlong]
         + [c_int] * 6 + [c_float, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p])
     sig("sglb_attn_prep_rows", [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_longlong]
@@ -319,6 +321,20 @@ def linear(x, w, bias=None, force_mode: int = -1, force_splits: int = 0, out=Non
     _check(lib().sglb_gemm_bf16(_p(x2), _p(w), _p(bias), _p(out), M, N, K, _p(sc.workspace), sc.bytes,
                                 _p(sc.counters), force_mode, force_splits, _stream()), "gemm_bf16")
     return out.view(*x.shape[:-1], N)
+
+
+def linear_part(x, w):
+    """`x [M, K] @ w [N, K]^T` where x is a column range of a wider product: its rows lie apart, and are read where they are."""
+    M, K = x.shape
+    N = w.shape[0]
+    if M == 0 or K % 8 or N % 8 or x.stride(1) != 1 or x.stride(0) % 8 or x.stride(0) < K or not w.is_contiguous() \
+            or x.data_ptr() % 16 or w.data_ptr() % 16:
+        return linear(x.contiguous(), w)
+    out = torch.empty((M, N), dtype=x.dtype, device=x.device)
+    sc = gemm_scratch(x.device)
+    _check(lib().sglb_gemm_bf16_ld(x.data_ptr(), x.stride(0), _p(w), None, _p(out), M, N, K, _p(sc.workspace), sc.bytes,
+                                   _p(sc.counters), _stream()), "gemm_bf16_ld")
+    return out
 
 
 def rope_qknorm_kvwrite(qkv, positions, cos_sin, q_norm_w, k_norm_w, eps, num_q_heads, num_kv_heads, head_dim,
@@ -903,9 +919,11 @@ def latent_extend(q, kv, k_rot, out, plan, dim, v_dim, scale, window=0, sink=Non
 
 # ---- gated delta rule over ragged batches (csrc/delta_scan.cu)
 def delta_scan(proj, g_off, b_off, a_off, conv_w, a_log, dt_bias, conv_state, state, slots, heads, kv_heads, dim, vdim,
-               cu=None, prefix=None, track_len=None, track_slot=None, lens=None, channel_a=None):
+               cu=None, prefix=None, track_len=None, track_slot=None, lens=None, channel_a=None, ba=None, grouped=None):
     """Read-outs fp32 `[T, heads, vdim]` of the rows of `proj [T, ld]` (columns `q | k | v` first, gate / beta / decay
-    inputs at the given offsets); windows and states of `slots` are updated in place.  `cu [B + 1]` / `prefix [B]`:
+    inputs at the given offsets, or those of `ba` if given); `grouped`: the columns of one q / k head and of the value heads that
+    use it, all neighbours, in a row that is `kv_heads` such groups (q, k and v first in each); then beta and decay inputs are
+    grouped as well, a group's betas first.  Windows and states of `slots` are updated in place.  `cu [B + 1]` / `prefix [B]`:
     ragged step (None: one row per request, all of them continuing); `lens`: its sequence lengths on the host, if known
     (without them the kernel for single tokens is launched on the chance that there are some).  `channel_a [T, heads * dim]`:
     one decay per head and key channel from these inputs, `dt_bias [heads * dim]` (`a_off` is not used then)."""
@@ -919,6 +937,14 @@ def delta_scan(proj, g_off, b_off, a_off, conv_w, a_log, dt_bias, conv_state, st
     gb = torch.empty((T, heads, 2), **f32)
     # coefficients of the chunks of 32 tokens: two 32 x 32 blocks and two vectors (sizes in csrc/delta_scan.cu)
     coef = torch.empty((T // 32 + 2 * B, heads, 2112), **f32) if cu is not None and singles != B else None
+    r = heads // kv_heads
+    ba = proj if ba is None else ba
+    assert ba.stride(1) == 1 and ba.dtype == proj.dtype and ba.shape[0] == T
+    if grouped is None:
+        cols = (0, kv_heads * dim, dim, 2 * kv_heads * dim, r * vdim, b_off, a_off, r)
+    else:
+        assert proj.shape[1] >= kv_heads * grouped and grouped >= 2 * dim + r * vdim
+        cols = (0, dim, grouped, 2 * dim, grouped, b_off, a_off, 2 * r)
     kq = gc = None
     if channel_a is not None:
         assert channel_a.is_contiguous() and channel_a.dtype == proj.dtype and channel_a.shape == (T, heads * dim)
@@ -927,21 +953,22 @@ def delta_scan(proj, g_off, b_off, a_off, conv_w, a_log, dt_bias, conv_state, st
             kq = torch.empty((T, heads, 3, dim), **f32)
             gc = torch.empty((T // 32 + 2 * B, heads, dim), **f32)
     o = torch.empty((T, heads, vdim), **f32)
-    _check(lib().sglb_delta_scan(_p(proj), proj.stride(0), g_off, b_off, a_off, _p(conv_w), _p(a_log), _p(dt_bias),
+    _check(lib().sglb_delta_scan(_p(proj), proj.stride(0), _p(ba), ba.stride(0), (c_int * 8)(*cols), _p(conv_w), _p(a_log), _p(dt_bias),
                                  _p(channel_a), _p(conv_state), _p(state), _p(slots), _p(cu), _p(prefix), _p(track_len),
                                  _p(track_slot), _p(qk), _p(v), _p(gb), _p(coef), _p(kq), _p(gc), _p(o), B, T, heads,
                                  kv_heads, dim, vdim, conv_w.shape[1], singles, _f32(proj), _stream()), "delta_scan")
     return o
 
 
-def delta_gate(o, gate, weight, eps, act="silu"):
+def delta_gate(o, gate, weight, eps, act="silu", group=None, step=None):
     """`rmsnorm(o) * weight * act(gate)` per head, act silu or sigmoid: `o [T, H, V]` fp32, `gate [T, H * V]` (any row stride) -> `[T, H * V]`
-    in the gate's type."""
+    in the gate's type; `weight` fp32 or bf16.  `group`, `step`: the gates of every `group` heads are neighbours, those of the next
+    ones `step` columns further on."""
     T, H, V = o.shape
-    assert o.is_contiguous() and gate.stride(-1) == 1 and weight.dtype == torch.float32
+    assert o.is_contiguous() and gate.stride(-1) == 1 and weight.dtype in (torch.float32, torch.bfloat16) and weight.is_contiguous()
     out = torch.empty((T, H * V), dtype=gate.dtype, device=o.device)
-    _check(lib().sglb_delta_gate(_p(o), gate.data_ptr(), gate.stride(0), _p(weight), _p(out), T, H, V, float(eps),
-                                 int(act == "sigmoid"), _f32(gate), _stream()), "delta_gate")
+    _check(lib().sglb_delta_gate(_p(o), gate.data_ptr(), gate.stride(0), group or H, step or H * V, _p(weight), _f32(weight), _p(out),
+                                 T, H, V, float(eps), int(act == "sigmoid"), _f32(gate), _stream()), "delta_gate")
     return out
 
 
