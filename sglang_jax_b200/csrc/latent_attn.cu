@@ -5,6 +5,7 @@
 //                     and the queries' rotary part (interleaved pairs, fp32 angles), writes the cache rows; where queries
 //                     have a latent of their own, RMS-normalises that instead, and
 //   latent_rotate     rotates the queries that come out of it
+//   mla_prep          the same pass for a step whose latent and queries come from projections of their own
 //   latent_attn_any   absorbed attention of single query tokens on the CUDA cores, everything in fp32: the fp32 mode,
 //                     and bf16 sizes that the tensor-core kernels (mla.cu, latent_extend.cu) do not take; window, sink
 //   latent_gather     cache rows of whole sequences (or from a token on) -> contiguous latents and key parts (input of the
@@ -134,6 +135,73 @@ latent_prep_kernel(T* __restrict__ proj, long long ld, int q_off, int dkv_off, i
     T* q = row + q_off + static_cast<long long>(h) * (dim + rot) + dim + 2 * i;
     rotate_pairs<T, VEC>(q, q, cs, half, i);
   }
+}
+
+// 8 lanes of a rotary part of `2 * half` lanes: interleaved pairs of lanes, or (SPLIT) lane i with lane i + half; cs = [cos | sin]
+// of the position, null: no rotation.  Unit u of `half / 4` (SPLIT: half / 8, two vectors each).
+template <bool SPLIT>
+__device__ __forceinline__ void rotate_unit(const __nv_bfloat16* src, __nv_bfloat16* dst, const float* __restrict__ cs, int half, int u) {
+  using V = Vec<__nv_bfloat16, 8>;
+  if constexpr (SPLIT) {
+    V a = *reinterpret_cast<const V*>(src + 8 * u), b = *reinterpret_cast<const V*>(src + half + 8 * u);
+    if (cs != nullptr) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float x = to_f(a.v[e]), y = to_f(b.v[e]), c = cs[8 * u + e], s = cs[half + 8 * u + e];
+        a.v[e] = from_f<__nv_bfloat16>(x * c - y * s);
+        b.v[e] = from_f<__nv_bfloat16>(y * c + x * s);
+      }
+    }
+    *reinterpret_cast<V*>(dst + 8 * u) = a;
+    *reinterpret_cast<V*>(dst + half + 8 * u) = b;
+  } else if (cs != nullptr) {
+    rotate_pairs<__nv_bfloat16, 8>(src + 8 * u, dst + 8 * u, cs, half, 4 * u);
+  } else {
+    *reinterpret_cast<V*>(dst + 8 * u) = *reinterpret_cast<const V*>(src + 8 * u);
+  }
+}
+
+// One CTA per token, bf16, 16-byte accesses throughout.  Reads the latent's row `[R | rot]` once and writes the cache row; the
+// queries' rotary lanes are rotated where the projection left them, so that the attention kernels read them in place.  Bound by
+// launch latency in decode (4 us at 96 tokens of 16 heads), by memory in prefill.  Eleven elementwise kernels and a scatter did this
+// before: 45 us a layer at 96 tokens.
+template <bool SPLIT>
+__global__ void __launch_bounds__(kPrepThreads)
+mla_prep_kernel(const __nv_bfloat16* __restrict__ lat, long long lat_ld, __nv_bfloat16* __restrict__ q, long long q_ld, int H,
+                int dim, int rot, int R, const __nv_bfloat16* __restrict__ norm_w, float w_add, float eps,
+                const float* __restrict__ cos_sin, const int* __restrict__ positions, const int* __restrict__ loc,
+                __nv_bfloat16* __restrict__ cache, int row_elems) {
+  __shared__ float red[kPrepThreads / 32];
+  pdl_wait();
+  const int t = blockIdx.x, tid = threadIdx.x, half = rot / 2;
+  const int units = rot / (SPLIT ? 16 : 8);
+  const float* cs = cos_sin != nullptr ? cos_sin + static_cast<long long>(positions[t]) * rot : nullptr;
+  const __nv_bfloat16* row = lat + static_cast<long long>(t) * lat_ld;
+  const float ss = squares<__nv_bfloat16, 8>(row, R);
+  if ((tid & 31) == 0) red[tid >> 5] = ss;
+  if (cs != nullptr) {
+    for (int j = tid; j < H * units; j += kPrepThreads) {
+      const int h = j / units;
+      __nv_bfloat16* p = q + static_cast<long long>(t) * q_ld + static_cast<long long>(h) * (dim + rot) + dim;
+      rotate_unit<SPLIT>(p, p, cs, half, j - h * units);
+    }
+  }
+  __syncthreads();
+  if (loc[t] < 0) return;
+  __nv_bfloat16* dst = cache + static_cast<long long>(loc[t]) * row_elems;
+  float tot = 0.f;
+#pragma unroll
+  for (int i = 0; i < kPrepThreads / 32; ++i) tot += red[i];
+  const float inv = 1.f / sqrtf(tot / R + eps);
+  using V = Vec<__nv_bfloat16, 8>;
+  for (int i = tid * 8; i < R; i += kPrepThreads * 8) {
+    V a = *reinterpret_cast<const V*>(row + i);
+    const V w = *reinterpret_cast<const V*>(norm_w + i);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) a.v[e] = from_f<__nv_bfloat16>(to_f(a.v[e]) * inv * (to_f(w.v[e]) + w_add));
+    *reinterpret_cast<V*>(dst + i) = a;
+  }
+  for (int u = kPrepThreads - 1 - tid; u < units; u += kPrepThreads) rotate_unit<SPLIT>(row + R, dst + R, cs, half, u);
 }
 
 // Rotates the last `rot` of every head's `dim + rot` lanes in place.
@@ -298,6 +366,27 @@ int sglb_latent_prep(void* proj, long long ld, int q_off, int dkv_off, int T, in
   if (is_f32) run(wide ? latent_prep_kernel<float, 4> : latent_prep_kernel<float, 1>, static_cast<float*>(proj));
   else run(wide ? latent_prep_kernel<__nv_bfloat16, 8> : latent_prep_kernel<__nv_bfloat16, 1>,
            static_cast<__nv_bfloat16*>(proj));
+  return static_cast<int>(cudaGetLastError());
+}
+
+// lat [T, lat_ld] = [latent (R) | key part (rot)], head h of token t's query at q + t * q_ld + h * (dim + rot), rotated in place; the
+// normalised latent (norm_w [R] + w_add) and the key part go to row loc[t] of the cache (< 0: nowhere).  cos_sin null: no
+// positions.  `split`: lane i of a rotary part turns with lane i + rot / 2 (else neighbours).  bf16; R, dim, lds and row_elems
+// whole 16-byte units.
+int sglb_mla_prep(const void* lat, long long lat_ld, void* q, long long q_ld, int T, int H, int dim, int rot, int R,
+                  const void* norm_w, float w_add, float eps, const float* cos_sin, int split, const int* positions,
+                  const int* loc, void* cache, int row_elems, cudaStream_t s) {
+  using namespace sglb;
+  if (T <= 0) return 0;
+  auto whole = [](long long v) { return v % 8 == 0; };
+  auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+  if (!whole(lat_ld) || !whole(q_ld) || !whole(dim) || !whole(R) || !whole(row_elems) || rot % (split ? 16 : 8) != 0 ||
+      row_elems < R + rot || H < 1 || !aligned(lat) || !aligned(q) || !aligned(norm_w) || !aligned(cache))
+    return -kBadArgument;
+  launch_pdl(split ? mla_prep_kernel<true> : mla_prep_kernel<false>, dim3(T), dim3(kPrepThreads), 0, s,
+             static_cast<const __nv_bfloat16*>(lat), lat_ld, static_cast<__nv_bfloat16*>(q), q_ld, H, dim, rot, R,
+             static_cast<const __nv_bfloat16*>(norm_w), w_add, eps, cos_sin, positions, loc,
+             static_cast<__nv_bfloat16*>(cache), row_elems);
   return static_cast<int>(cudaGetLastError());
 }
 

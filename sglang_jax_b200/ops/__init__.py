@@ -252,6 +252,14 @@ def latent_prep(proj, *a, **kw):
     return (_native() if use_native_wide(proj) else reference).latent_prep(proj, *a, **kw)
 
 
+def mla_prep_supported(q, *a) -> bool:
+    return use_native(q) and _native().mla_prep_supported(q, *a)
+
+
+def mla_prep(*a):
+    return _native().mla_prep(*a)
+
+
 def latent_rotate(q, *a):
     (_native() if use_native_wide(q) else reference).latent_rotate(q, *a)
 
@@ -365,6 +373,18 @@ def fused_experts(x, w13, w2, topk_weights, topk_ids, expert_start=0, workspace=
         return moe_native.fused_experts(x, w13, w2, topk_weights, topk_ids, expert_start, workspace, add)
     y = reference.moe_forward(x, w13, w2, topk_weights, topk_ids, expert_start)
     return y if add is None else (y.float() + add.float()).to(y.dtype)
+
+
+def mla_tokens_supported(q_pe, cache, heads: int, rank: int, page_size: int) -> bool:
+    """Whether single query tokens with latent queries `[T, heads, rank]` can go through `mla_tokens`."""
+    probe = q_pe.new_empty(0, heads, rank)
+    return use_native(q_pe) and _native().mla_decode_supported(probe, q_pe, cache, rank, page_size)
+
+
+def mla_tokens(q_latent, q_pe, cache, fb, scale, rows, lens):
+    """Absorbed attention of query tokens on their own, unrounded weights: query n sees the first `lens[n]` tokens of page-table
+    row `rows[n]`."""
+    return _native().mla_decode(q_latent, q_pe, cache, fb.page_table, rows, lens, fb.page_size, scale, fb.max_seq_len, exact=True)
 
 
 def mla_paged_attention(q_latent, q_pe, kv_buffer, page_table, req_pool_indices, seq_lens, page_size, scale,

@@ -115,6 +115,8 @@ def lib():
     sig("sglb_latent_prep", [c_void_p, c_longlong] + [c_int] * 7 + [c_void_p, c_float, c_void_p, c_void_p, c_void_p,
                                                                     c_void_p, c_int, c_void_p, c_int, c_void_p, c_int,
                                                                     c_void_p])
+    sig("sglb_mla_prep", [c_void_p, c_longlong, c_void_p, c_longlong] + [c_int] * 5 + [c_void_p, c_float, c_float, c_void_p, c_int,
+                          c_void_p, c_void_p, c_void_p, c_int, c_void_p])
     sig("sglb_latent_rotate", [c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p])
     sig("sglb_latent_attn_any", [c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p,
                                  c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_int, c_void_p])
@@ -861,6 +863,34 @@ def latent_prep(proj, q_off, dkv_off, heads, dim, rot, rank, norm_w, eps, cos_si
                                   cache.shape[-1], _p(q_latent), q_rank, _p(q_norm_w), _f32(proj), _stream()),
            "latent_prep")
     return q_latent
+
+
+def mla_prep_supported(q, latent, cache, norm_w, cos_sin, positions, loc, rank, split) -> bool:
+    """Whether `mla_prep` takes these tensors (`q [T, H, dim + rot]`, `latent [T, >= rank + rot]`)."""
+    rot = latent.shape[1] - rank
+    dim = q.shape[2] - rot
+    whole = lambda *v: all(n % 8 == 0 for n in v)
+    return (q.dtype == latent.dtype == cache.dtype == norm_w.dtype == torch.bfloat16 and rot > 0 and dim > 0
+            and whole(rank, dim, rot // 2 if split else rot, q.stride(0), latent.stride(0), cache.shape[-1])
+            and q.stride(2) == latent.stride(1) == 1 and q.stride(1) == q.shape[2] and q.stride(0) >= q.shape[1] * q.shape[2]
+            and cache.is_contiguous() and cache.shape[-1] >= rank + rot and norm_w.is_contiguous() and norm_w.numel() == rank
+            and all(t.data_ptr() % 16 == 0 for t in (q, latent, cache, norm_w))
+            and positions.dtype == loc.dtype == torch.int32 and positions.dim() == 1 and positions.is_contiguous()
+            and loc.is_contiguous() and positions.numel() >= q.shape[0] <= loc.numel()
+            and (cos_sin is None or (cos_sin.dtype == torch.float32 and cos_sin.is_contiguous() and cos_sin.shape[-1] == rot
+                                     and cos_sin.device == q.device))
+            and q.device == latent.device == cache.device == norm_w.device == positions.device == loc.device)
+
+
+def mla_prep(q, latent, norm_w, eps, gemma, cos_sin, split, positions, loc, cache):
+    """Rotates the last lanes of every head of `q` in place (`cos_sin` None: no positions) and writes the normalised latent and
+    the rotated key part of `latent [T, rank + rot]` into `cache [pages, P, row]` at slots `loc`.  `split`: a lane turns with the
+    one half a rotary part away, else with its neighbour."""
+    rank = norm_w.numel()
+    rot = latent.shape[1] - rank
+    _check(lib().sglb_mla_prep(latent.data_ptr(), latent.stride(0), q.data_ptr(), q.stride(0), q.shape[0], q.shape[1],
+                               q.shape[2] - rot, rot, rank, _p(norm_w), 1.0 if gemma else 0.0, float(eps), _p(cos_sin),
+                               int(split), _p(positions), _p(loc), _p(cache), cache.shape[-1], _stream()), "mla_prep")
 
 
 def latent_rotate(q, dim, cos_sin, positions):
