@@ -31,13 +31,13 @@ ACCURATE = {"residual_stream.cu", "latent_attn.cu", "delta_scan.cu", "window_att
 # what one model family launches outside sampling: enough for a library of its own, which a fresh checkout builds in a
 # few seconds (`ops/native.py: prefer_kernel_set`)
 KERNEL_SETS = {
-    "latent_delta": ["runtime.cu", "gemm_sm100.cu", "mla.cu", "latent_attn.cu", "latent_extend.cu", "delta_scan.cu",
+    "latent_delta": ["runtime.cu", "gemm_sm100.cu", "gemm_pair.cu", "mla.cu", "latent_attn.cu", "latent_extend.cu", "delta_scan.cu",
                      "residual_stream.cu"],
-    "window_delta": ["runtime.cu", "gemm_sm100.cu", "window_attn.cu", "window_extend.cu", "delta_scan.cu",
+    "window_delta": ["runtime.cu", "gemm_sm100.cu", "gemm_pair.cu", "window_attn.cu", "window_extend.cu", "delta_scan.cu",
                      "residual_stream.cu", "moe.cu", "moe_any.cu"],
-    "window_latent": ["runtime.cu", "gemm_sm100.cu", "window_attn.cu", "window_extend.cu", "mla.cu", "latent_attn.cu",
+    "window_latent": ["runtime.cu", "gemm_sm100.cu", "gemm_pair.cu", "window_attn.cu", "window_extend.cu", "mla.cu", "latent_attn.cu",
                       "latent_extend.cu", "residual_stream.cu", "moe.cu", "moe_any.cu"],
-    "chunk_ssd": ["runtime.cu", "gemm_sm100.cu", "window_attn.cu", "window_extend.cu", "ssd_scan.cu", "residual_stream.cu",
+    "chunk_ssd": ["runtime.cu", "gemm_sm100.cu", "gemm_pair.cu", "window_attn.cu", "window_extend.cu", "ssd_scan.cu", "residual_stream.cu",
                   "moe.cu", "moe_any.cu"],
 }
 

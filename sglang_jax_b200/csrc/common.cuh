@@ -329,6 +329,14 @@ __device__ __forceinline__ void multimem_st_v4(void* mc_addr, const uint4& v) {
                : "memory");
 }
 
+// One lane of a converged warp.  Roles of a single thread begin with this and not with `lane == 0`: the compiler then knows that one
+// thread runs them, and feeds tensor and copy instructions from uniform registers without asking which lanes are there.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r)::"memory");
+  return r != 0;
+}
+
 // named barrier among a subset of the CTA's warps
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
@@ -368,5 +376,9 @@ bool encode_tmap_2d(CUtensorMap* out, const void* base, uint64_t inner_elems, ui
                     uint32_t box_inner, uint32_t box_rows, int elem_bytes);
 bool encode_tmap_3d(CUtensorMap* out, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t stride1,
                     uint64_t stride2, uint32_t box_rows);
+// bf16 tensor of `rank` <= 4 dimensions, the first of 64 elements (128-byte swizzle), the others by byte strides (multiples of 16).
+// Elements outside the extents are read as zeros.
+bool encode_tmap_blocks(CUtensorMap* out, const void* base, int rank, const uint64_t* dims, const uint64_t* strides,
+                        const uint32_t* box);
 int sm_count();
 }  // namespace sglb

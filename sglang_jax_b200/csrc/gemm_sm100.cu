@@ -9,7 +9,8 @@
 // i overlaps the main loop of tile i+1.
 //
 // Two operand assignments share the kernel:
-//   MODE 0 ("tokens on M")   A = x tile (128 tokens), B = w tile (BN outputs).  Prefill.
+//   MODE 0 ("tokens on M")   A = x tile (128 tokens), B = w tile (BN outputs).  Prefill of what gemm_pair.cu does not take:
+//          fp8, products fused with a collective, K that is no multiple of 64.
 //   MODE 1 ("weights on M")  A = w tile (128 outputs), B = x (all tokens, BN >= M).  Decode:
 //          the 128-row MMA dimension is filled with weight rows, so a batch of 1..256 tokens
 //          wastes no tensor-core rows, weights are streamed exactly once, and K is split over
@@ -27,6 +28,7 @@
 
 #include "common.cuh"
 #include "gemm_noalloc.h"
+#include "gemm_pair.h"
 
 namespace sglb {
 namespace {
@@ -1111,6 +1113,11 @@ int sglb_gemm_bf16_impl(const void* x, const void* w, const void* bias, void* ou
   }();
   int mode = force_mode >= 0 ? force_mode : (M <= 256 ? decode_mode : 0);
   if (mode == 1 && M > 256) mode = 0;
+  // Prefill sizes run on pairs of SMs (figures there).  Its maps split K into blocks of 64, so other K stay with the tiles below, as do
+  // fp8 operands and products fused with a collective; up to 256 tokens the weights are the only traffic that counts, and every SM
+  // streams an equal share of them (128 tokens, 5120 -> 51200: 109 us here, 112 us in pairs).
+  if (force_mode < 0 && M > 256 && K % BK == 0 && !fp8 && fused == nullptr && rs_world == 0)
+    return gemm_pair(x, ldx, w, bias, out, M, N, K, false, nullptr, 0, stream);
 
   Params p{};
   p.out = static_cast<__nv_bfloat16*>(out);

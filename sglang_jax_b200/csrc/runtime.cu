@@ -100,6 +100,24 @@ bool encode_tmap_3d(CUtensorMap* out, const void* base, uint64_t d0, uint64_t d1
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+bool encode_tmap_blocks(CUtensorMap* out, const void* base, int rank, const uint64_t* dims, const uint64_t* strides,
+                        const uint32_t* box) {
+  EncodeFn enc = get_encode();
+  if (!enc || rank < 2 || rank > 4 || (reinterpret_cast<uintptr_t>(base) & 15)) return false;
+  cuuint64_t d[4], st[3];
+  cuuint32_t b[4], estr[4] = {1, 1, 1, 1};
+  for (int i = 0; i < rank; ++i) {
+    d[i] = dims[i];
+    b[i] = box[i];
+    if (i + 1 < rank) {
+      if (strides[i] & 15) return false;
+      st[i] = strides[i];
+    }
+  }
+  return enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(base), d, st, b, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 }  // namespace sglb
 
 extern "C" {

@@ -62,6 +62,7 @@ def lib():
     sig("sglb_gemm_max_counters", [c_int])
     sig("sglb_gemm_bf16", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_size_t,
                                  c_void_p, c_int, c_int, c_void_p])
+    sig("sglb_gemm_pair", [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p] + [c_int] * 5 + [c_void_p])
     sig("sglb_gemm_bf16_ld", [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_size_t,
                               c_void_p, c_void_p])
     sig("sglb_rmsnorm", [c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_float, c_int, c_void_p])
@@ -323,6 +324,18 @@ def linear(x, w, bias=None, force_mode: int = -1, force_splits: int = 0, out=Non
     _check(lib().sglb_gemm_bf16(_p(x2), _p(w), _p(bias), _p(out), M, N, K, _p(sc.workspace), sc.bytes,
                                 _p(sc.counters), force_mode, force_splits, _stream()), "gemm_bf16")
     return out.view(*x.shape[:-1], N)
+
+
+def gemm_pair(x, w, bias=None, gated: bool = False, tile: int = 0):
+    """`x [T, K] @ w [N, K]^T (+ bias)` on pairs of SMs; K a multiple of 64, rows of x any whole 16-byte units apart.  `gated`: the
+    halves of w are gate and up rows, the result `silu(x gate^T) * (x up^T)`, from the fp32 sums.  `tile`: tokens of a tile (0: by
+    the sizes)."""
+    T, K = x.shape
+    N = w.shape[0] // 2 if gated else w.shape[0]
+    assert x.stride(1) == 1 and w.is_contiguous() and w.shape[1] == K
+    out = torch.empty((T, N), dtype=x.dtype, device=x.device)
+    _check(lib().sglb_gemm_pair(x.data_ptr(), x.stride(0), _p(w), _p(bias), _p(out), T, N, K, int(gated), tile, _stream()), "gemm_pair")
+    return out
 
 
 def linear_part(x, w):
