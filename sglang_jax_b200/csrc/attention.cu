@@ -241,7 +241,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmap, const AttnParams p
   float* merge = reinterpret_cast<float*>(smem);   // reused after the main loop
 
   const int b = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int G = p.Hq / p.Hkv;
   pdl_wait();
   const int seq = p.seq_lens[b];
@@ -269,7 +269,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tmap, const AttnParams p
   WarpState<D> st;
   st.init();
   if (warp == kConsumerWarps) {
-    if (lane == 0) {
+    if (elect_one()) {
       prefetch_tmap(&tmap);
       int stage = 0;
       uint32_t phase = 0;
@@ -435,7 +435,7 @@ paged_extend_kernel(const __grid_constant__ CUtensorMap tmap, const AttnParams p
   const int hq = blockIdx.y;
   const int G = p.Hq / p.Hkv;
   const int kvh = hq / G;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int q_begin = p.cu_q_lens[b];
   const int q_len = p.cu_q_lens[b + 1] - q_begin;
   const int prefix = p.prefix_lens[b];
@@ -461,7 +461,7 @@ paged_extend_kernel(const __grid_constant__ CUtensorMap tmap, const AttnParams p
   __syncthreads();
 
   if (warp == kConsumerWarps) {
-    if (lane == 0) {
+    if (elect_one()) {
       prefetch_tmap(&tmap);
       int stage = 0;
       uint32_t phase = 0;
@@ -651,7 +651,7 @@ paged_extend_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const __grid
   }
   const int hq = blockIdx.y;
   const int kvh = hq / (p.Hq / p.Hkv);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int q_begin = p.cu_q_lens[b];
   const int q_len = p.cu_q_lens[b + 1] - q_begin;
   const int prefix = p.prefix_lens[b];
@@ -691,7 +691,7 @@ paged_extend_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const __grid
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0 && elect_one()) {
       const uint32_t qb = smem_u32(&bars->q_full);
       mbar_expect_tx(qb, kQBytes);
       tma_load_2d(smem_u32(q_s), &tmap_q, qb, hq * HD, q_begin + q0);
@@ -733,7 +733,7 @@ paged_extend_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const __grid
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0 && elect_one()) {
       constexpr uint32_t idesc_s = make_idesc(BQ2, BKV, 1, 1);                  // Q (K-major) x K (K-major)
       constexpr uint32_t idesc_pv = make_idesc(BQ2, HD, 1, 1) | (1u << 16);     // P (K-major) x V (MN-major)
       bool ok = mbar_wait(smem_u32(&bars->q_full), 0);

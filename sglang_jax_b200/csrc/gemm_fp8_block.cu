@@ -95,7 +95,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   uint64_t* acc_empty = acc_full + kAccBufs;     // [kAccBufs] ... and has been read out again
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + kAccBufs);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     prefetch_tmap(&tmap_a);
@@ -122,7 +122,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   pdl_wait();
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0, it = 0;
       uint32_t phase = 0;
       BTile t;
@@ -146,7 +146,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc(BM, BN, 0, 0);
       int stage = 0, it = 0, buf = 0;
       uint32_t phase = 0, buf_phase = 0;

@@ -92,7 +92,7 @@ latent_extend_kernel(const __grid_constant__ CUtensorMap map_qn, const __grid_co
     if (tile < 0) return;
   }
   const int head = blockIdx.y;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int q_len = p.q_len[b], prefix = p.prefix[b], seq = prefix + q_len, ctx0 = p.ctx_start[b] - (p.skip != nullptr ? p.skip[b] : 0);
   const int q0 = tile * kTiles * kTileQ;
   const KeyTiles<kTileK> keys(p.win, prefix + q0, prefix + min(q0 + kTiles * kTileQ, q_len) - 1);
@@ -134,7 +134,7 @@ latent_extend_kernel(const __grid_constant__ CUtensorMap map_qn, const __grid_co
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t qb = smem_u32(&bars->q_full);
       mbar_expect_tx(qb, kTiles * nb_q * kBlkQ);
       for (int t = 0; t < kTiles; ++t) {
@@ -174,7 +174,7 @@ latent_extend_kernel(const __grid_constant__ CUtensorMap map_qn, const __grid_co
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = make_idesc(kTileQ, kTileK, 1, 1);
       const uint32_t idesc_pv = make_idesc(kTileQ, 64 * p.nb_v, 1, 1) | (1u << 16);      // B (values) is MN-major
       const int steps_n = (p.dim + 15) / 16, steps_r = (p.rot + 15) / 16;

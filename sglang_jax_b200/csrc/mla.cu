@@ -92,7 +92,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
   volatile int* abort_flag = reinterpret_cast<volatile int*>(empty_bar + kMaxStages);
 
   const int b = blockIdx.x, hg = blockIdx.y, split = blockIdx.z;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int seq = p.seq_lens[b];
   const int* pt_row = p.page_table + static_cast<size_t>(p.req_pool_indices[b]) * p.max_pages;
   const int first = p.window > 0 && seq > p.window ? seq - p.window : 0;      // first visible token
@@ -113,7 +113,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
 
   if (warp == kConsumerWarps) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       prefetch_tmap(&tmap);
       const uint64_t pol = l2_policy_evict_first();      // every latent row is read once per head group
       int stage = 0;
