@@ -5,7 +5,6 @@ biased, grouped and biased-grouped selection, renormalisation, `routed_scaling_f
 from __future__ import annotations
 
 import torch
-import torch.nn.functional as F
 from torch import nn
 
 from .. import ops
@@ -33,7 +32,7 @@ class GateLogit(nn.Module):
         param.data.copy_(w)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        return F.linear(x.float(), self.weight.float(), self.bias.float() if self.bias is not None else None)
+        return ops.router_logits(x, self.weight, self.bias)
 
     def route_by_logit(self, x: torch.Tensor, top_k: int):
         """The experts with the largest logits, weights the softmax over the chosen logits only: `(weights fp32, ids int32)`,

@@ -226,6 +226,15 @@ def low_rank_up(x, w):
     return reference.linear(x, w)
 
 
+def router_logits(x, weight, bias=None):
+    """`x weight^T + bias` in fp32, whatever the operands' type."""
+    if use_native(x):
+        from . import moe_native
+        if moe_native.router_logits_supported(x, weight, bias):
+            return moe_native.router_logits(x, weight, bias)
+    return reference.linear(x.float(), weight.float(), bias.float() if bias is not None else None)
+
+
 def route_by_logit(x, weight, bias, top_k):
     """The `top_k` experts with the largest logits `x weight^T + bias` (fp32) and the softmax over them."""
     if use_native_wide(x) and weight.shape[0] <= 512 and top_k <= 16 and weight.dtype == x.dtype:

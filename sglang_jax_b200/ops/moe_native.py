@@ -2,7 +2,7 @@
 
 from __future__ import annotations
 
-from ctypes import c_float, c_int, c_size_t, c_void_p
+from ctypes import c_float, c_int, c_longlong, c_size_t, c_void_p
 
 import torch
 
@@ -17,7 +17,9 @@ def _lib():
     if not _bound:
         L.sglb_topk_route.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                       c_int, c_int, c_float, c_void_p]
-        L.sglb_moe_align.argtypes = [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
+        L.sglb_router_logits.argtypes = [c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]
+        L.sglb_gemm_pair_grouped.argtypes = [c_void_p] * 7 + [c_int] * 6 + [c_void_p]
+        L.sglb_moe_align.argtypes = [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                      c_void_p, c_void_p, c_void_p, c_void_p]
         L.sglb_moe_gather.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p]
         L.sglb_moe_combine.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]
@@ -54,8 +56,28 @@ def topk_route(router_logits, top_k, scoring="softmax", renormalize=True, correc
     return w, ids
 
 
+def router_logits_supported(x, weight, bias=None) -> bool:
+    return (x.dim() == 2 and x.dtype == weight.dtype == torch.bfloat16 and weight.is_contiguous() and x.shape[1] % 32 == 0
+            and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.stride(0) >= x.shape[1] and x.data_ptr() % 16 == 0
+            and weight.data_ptr() % 16 == 0 and x.device == weight.device
+            and (bias is None or (bias.dtype == torch.bfloat16 and bias.is_contiguous())))
+
+
+def router_logits(x, weight, bias=None):
+    """`x [T, K] @ weight [E, K]^T (+ bias)` in fp32 arithmetic from bf16 operands."""
+    T, K = x.shape
+    out = torch.empty((T, weight.shape[0]), dtype=torch.float32, device=x.device)
+    native._check(_lib().sglb_router_logits(out.data_ptr(), x.data_ptr(), x.stride(0), weight.data_ptr(), native._p(bias), T,
+                                            weight.shape[0], K, native._stream()), "router_logits")
+    return out
+
+
+# rows of a token tile in the lists of `moe_align`, where a kernel does not want others
+TILE_ROWS = 128
+
+
 class MoeWorkspace:
-    """Index buffers of one MoE layer call, sized for `max_pairs` routed (token, expert) pairs."""
+    """Index buffers of one MoE layer call, sized for `max_pairs` routed (token, expert) pairs and tiles of at least 32 rows."""
 
     def __init__(self, max_pairs: int, num_local_experts: int, device):
         self.max_pairs = max_pairs
@@ -63,14 +85,17 @@ class MoeWorkspace:
         self.offsets = torch.zeros(num_local_experts + 1, **i32)
         self.pair_row = torch.empty(max_pairs, **i32)
         self.row_token = torch.empty(max_pairs, **i32)
-        self.tile_group = torch.empty(max_pairs // 128 + num_local_experts + 1, **i32)
-        self.tile_row0 = torch.empty(max_pairs // 128 + num_local_experts + 1, **i32)
+        self.tile_group = torch.empty(max_pairs // 32 + num_local_experts + 1, **i32)
+        self.tile_row0 = torch.empty(max_pairs // 32 + num_local_experts + 1, **i32)
+        self.tile_rows = TILE_ROWS
         self.counts = torch.zeros(2, **i32)
 
 
-def moe_align(topk_ids, expert_start, num_local_experts, ws: MoeWorkspace, expert_hist=None):
+def moe_align(topk_ids, expert_start, num_local_experts, ws: MoeWorkspace, expert_hist=None, tile_rows: int = TILE_ROWS):
     T, k = topk_ids.shape
-    rc = _lib().sglb_moe_align(topk_ids.data_ptr(), T * k, k, expert_start, num_local_experts, ws.offsets.data_ptr(),
+    assert tile_rows >= 32
+    ws.tile_rows = tile_rows
+    rc = _lib().sglb_moe_align(topk_ids.data_ptr(), T * k, k, expert_start, num_local_experts, tile_rows, ws.offsets.data_ptr(),
                                ws.pair_row.data_ptr(), ws.row_token.data_ptr(), ws.tile_group.data_ptr(),
                                ws.tile_row0.data_ptr(), ws.counts.data_ptr(),
                                expert_hist.data_ptr() if expert_hist is not None else None, native._stream())
@@ -86,9 +111,41 @@ def moe_gather(x, ws: MoeWorkspace, max_rows: int):
     return out
 
 
+def on_pairs(rows: int, K: int) -> bool:
+    """Whether a grouped product of `rows` rows runs on pairs of SMs (`csrc/gemm_pair.cu`): its maps want whole blocks of 64 lanes.  Up
+    to 256 rows the weights' bytes are shared out evenly over all SMs instead."""
+    return rows > 256 and K % 64 == 0
+
+
+def pair_tile(rows: int, experts: int) -> int:
+    """Rows of a token tile for `rows` pairs over `experts`: an expert's rows in one tile where 256 hold them (with a quarter to
+    spare, as tokens are not spread evenly: a second tile reads all of the weights again), else in few of equal size.
+    Both products of 64 experts of 768 x 2048, tiles of 64 / 128 / 192 / 256: 182 / 158 / 154 / 154 us at 1024 tokens x 8, 304 / 232 / 215
+    / 223 at 2500, 387 / 271 / 248 / 243 at 3000; in 128-row tiles of single SMs with the activation of its own 180, 275 and 315."""
+    mean = max(rows // max(experts, 1), 1)
+    n = -(-mean // 256)
+    return min(256, -(-mean * 5 // (4 * n * 32)) * 32)
+
+
+def grouped_gemm_pair(x_sorted, w, ws: MoeWorkspace, rows: int, gated: bool = False):
+    """`grouped_gemm` on pairs of SMs; `gated`: `w [E_local, 2 N, K]` holds gate, then up rows, the result is `silu(gate) * up` of the
+    fp32 sums."""
+    E, N, K = w.shape
+    N //= 2 if gated else 1
+    out = torch.empty((rows, N), dtype=x_sorted.dtype, device=x_sorted.device)
+    rc = _lib().sglb_gemm_pair_grouped(x_sorted.data_ptr(), w.data_ptr(), out.data_ptr(), ws.offsets.data_ptr(), ws.tile_group.data_ptr(),
+                                       ws.tile_row0.data_ptr(), ws.counts.data_ptr() + 4, rows, N, K, E, int(gated), ws.tile_rows,
+                                       native._stream())
+    native._check(rc, "gemm_pair_grouped")
+    return out
+
+
 def grouped_gemm(x_sorted, w, ws: MoeWorkspace, rows: int):
     """`x_sorted [rows, K]` (rows sorted by expert), `w [E_local, N, K]` -> `[rows, N]`."""
     E, N, K = w.shape
+    if on_pairs(rows, K):
+        return grouped_gemm_pair(x_sorted, w, ws, rows)
+    assert ws.tile_rows == TILE_ROWS or rows <= 256
     out = torch.empty((rows, N), dtype=x_sorted.dtype, device=x_sorted.device)
     sc = native.gemm_scratch(x_sorted.device)
     rc = _lib().sglb_grouped_gemm_bf16(x_sorted.data_ptr(), w.data_ptr(), out.data_ptr(), ws.offsets.data_ptr(),
@@ -196,10 +253,12 @@ def fused_experts(x, w13, w2, topk_weights, topk_ids, expert_start: int = 0, ws:
     pairs = T * k
     if ws is None or ws.max_pairs < pairs:
         ws = MoeWorkspace(pairs, E_local, x.device)
-    moe_align(topk_ids, expert_start, E_local, ws)
-    xs = moe_gather(x, ws, pairs)
-    h = grouped_gemm(xs, w13, ws, pairs)
-    a = native.silu_and_mul(h)
+    if on_pairs(pairs, H) and on_pairs(pairs, w2.shape[2]):
+        moe_align(topk_ids, expert_start, E_local, ws, tile_rows=pair_tile(pairs, E_local))
+        a = grouped_gemm_pair(moe_gather(x, ws, pairs), w13, ws, pairs, gated=True)
+    else:
+        moe_align(topk_ids, expert_start, E_local, ws)
+        a = native.silu_and_mul(grouped_gemm(moe_gather(x, ws, pairs), w13, ws, pairs))
     y = grouped_gemm(a, w2, ws, pairs)
     return moe_combine(y, topk_weights, ws, T, add=add, out=out)
 
