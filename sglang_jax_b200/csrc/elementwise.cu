@@ -213,103 +213,197 @@ __global__ void argmax_kernel(int* __restrict__ out, const T* __restrict__ logit
   }
 }
 
-// One warp per (token, head) of the fused qkv row:
-//   q heads: optional RMSNorm over the head, RoPE, -> q_out[t, h, :]
-//   k heads: optional RMSNorm, RoPE, -> cache[page, 0, h, off, :]
-//   v heads: -> cache[page, 1, h, off, :]
-// Lane l holds elements l, l+32, l+64, ... of the head, so the neox partner i + rd/2 of an element
-// lives in the same lane (rd/2 is a multiple of 32).
 #ifdef SGLB_BOUNDS_CHECK
 // Checked build only: the extent of the KV buffers and where to report, set by sglb_debug_set_kv_pages().
 __device__ int g_dbg_kv_pages = 0;
 __device__ Status* g_dbg_status = nullptr;
 #endif
 
+// Every (token, head) of a step's queries, keys and values:
+//   q heads: optional RMSNorm over the head, RoPE, -> q_out[t, h, :]
+//   k heads: optional RMSNorm, RoPE, -> cache[page, 0, h, off, :]
+//   v heads: -> cache[page, 1, h, off, :]
+struct RopeParams {
+  __nv_bfloat16* q_out;
+  const __nv_bfloat16 *q, *k, *v;            // head h of token t at q + t * q_ts + h * q_hs, k + t * k_ts + h * D, v likewise
+  long long q_ts, k_ts, v_ts;
+  int q_hs;
+  const int* positions;
+  const float* cos_sin;                      // [position][cos | sin], rd / 2 each; null: no rotation
+  const __nv_bfloat16 *q_w, *k_w;            // norm weights (+ w_add) or null
+  float w_add, eps;
+  int Hq, Hkv, rd;
+  __nv_bfloat16* kv;
+  const int* loc;
+  int page_size;
+};
+
+// One CTA per token (and share of its heads where tokens are few): D / 8 lanes hold a head, 16 bytes each, lane u of the first half of the
+// rotary part turns with lane u + rd / 16.  A thread keeps its cosines, sines and norm weights for all heads that it takes.  Bound by
+// memory: 8192 tokens of 64 + 2 x 8 heads 230 us with 2-byte accesses and a position's row read again for every head, now 135.
+constexpr int kRopeThreads = 256;
+
 template <int D>
-__global__ void rope_qknorm_kvwrite_kernel(__nv_bfloat16* __restrict__ q_out, const __nv_bfloat16* __restrict__ qkv,
-                                           const int* __restrict__ positions, const float* __restrict__ cos_sin,
-                                           const __nv_bfloat16* __restrict__ q_w, const __nv_bfloat16* __restrict__ k_w,
-                                           float eps, long long T, int Hq, int Hkv, int rd,
-                                           __nv_bfloat16* __restrict__ kv, const int* __restrict__ loc, int page_size,
-                                           int is_neox) {
+__global__ void __launch_bounds__(kRopeThreads)
+rope_qknorm_kvwrite_kernel(const RopeParams p) {
+  constexpr int L = D / 8, kSlots = kRopeThreads / L;
+  const int t = blockIdx.x, u = threadIdx.x % L, lane = threadIdx.x & 31;
+  const int heads = p.Hq + 2 * p.Hkv, half = p.rd / 16;          // vectors in a half
+  pdl_wait();
+  const bool first = u < half, turns = p.cos_sin != nullptr && u < 2 * half;
+  const int partner = lane - u + (first ? u + half : u - half);
+  float c[8], sn[8];
+  if (turns) {
+    const float* cs = p.cos_sin + static_cast<long long>(p.positions[t]) * p.rd + 8 * (first ? u : u - half);
+#pragma unroll
+    for (int e = 0; e < 8; e += 4) {
+      const float4 a = *reinterpret_cast<const float4*>(cs + e), b = *reinterpret_cast<const float4*>(cs + p.rd / 2 + e);
+      c[e] = a.x, c[e + 1] = a.y, c[e + 2] = a.z, c[e + 3] = a.w;
+      sn[e] = b.x, sn[e + 1] = b.y, sn[e + 2] = b.z, sn[e + 3] = b.w;
+    }
+    if (first) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) sn[e] = -sn[e];
+    }
+  }
+  uint4 wq = make_uint4(0, 0, 0, 0), wk = wq;
+  if (p.q_w != nullptr) wq = reinterpret_cast<const uint4*>(p.q_w)[u];
+  if (p.k_w != nullptr) wk = reinterpret_cast<const uint4*>(p.k_w)[u];
+  long long slot_at = -1;
+  if (p.kv != nullptr) {
+    const int slot = p.loc[t];
+    const int page = slot / p.page_size, off = slot - page * p.page_size;
+    if (slot >= 0) slot_at = (static_cast<long long>(page) * 2 * p.Hkv * p.page_size + off) * D;
+#ifdef SGLB_BOUNDS_CHECK
+    if (g_dbg_kv_pages > 0 && (slot < 0 || page >= g_dbg_kv_pages)) {
+      if (threadIdx.x == 0) report(g_dbg_status, kOutOfBounds, t, slot);
+      slot_at = -1;
+    }
+#endif
+  }
+  // (all lanes of a warp stay in the loop together: they exchange values)
+  for (int h0 = blockIdx.y * kSlots; h0 < heads; h0 += gridDim.y * kSlots) {
+    const int h = h0 + threadIdx.x / L;
+    const bool is_q = h < p.Hq, is_k = !is_q && h < p.Hq + p.Hkv, in = h < heads;
+    const int hk = is_k ? h - p.Hq : h - p.Hq - p.Hkv;
+    const __nv_bfloat16* src = is_q ? p.q + t * p.q_ts + static_cast<long long>(h) * p.q_hs
+                                    : (is_k ? p.k + t * p.k_ts : p.v + t * p.v_ts) + static_cast<long long>(hk) * D;
+    uint4 raw = make_uint4(0, 0, 0, 0);
+    if (in) raw = reinterpret_cast<const uint4*>(src)[u];
+    const bool norm = is_q ? p.q_w != nullptr : is_k && p.k_w != nullptr;
+    if (p.q_w != nullptr || p.k_w != nullptr) {
+      float v[8], w[8], ss = 0.f;
+      unpack8(raw, v);
+      unpack8(is_q ? wq : wk, w);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ss += v[e] * v[e];
+#pragma unroll
+      for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      const float inv = rsqrtf(ss / D + p.eps);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = v[e] * inv * (w[e] + p.w_add);
+      if (norm) raw = pack8(v);                // rounded like the norm on its own, before the rotation
+    }
+    if (p.cos_sin != nullptr) {
+      const uint4 other = make_uint4(__shfl_sync(0xffffffffu, raw.x, partner), __shfl_sync(0xffffffffu, raw.y, partner),
+                                     __shfl_sync(0xffffffffu, raw.z, partner), __shfl_sync(0xffffffffu, raw.w, partner));
+      if (turns && (is_q || is_k)) {
+        float v[8], o[8];
+        unpack8(raw, v);
+        unpack8(other, o);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = v[e] * c[e] + o[e] * sn[e];
+        raw = pack8(v);
+      }
+    }
+    if (!in) continue;
+    if (is_q) {
+      reinterpret_cast<uint4*>(p.q_out + (static_cast<long long>(t) * p.Hq + h) * D)[u] = raw;
+    } else if (slot_at >= 0) {
+      const long long head = static_cast<long long>(is_k ? hk : hk + p.Hkv) * p.page_size * D;
+      reinterpret_cast<uint4*>(p.kv + slot_at + head)[u] = raw;
+    }
+  }
+}
+
+// The same for rotations of neighbouring lanes: one warp per (token, head), lane l holds elements l, l + 32, l + 64, ...
+template <int D>
+__global__ void rope_pairs_kernel(const RopeParams p, long long T) {
   pdl_wait();
   constexpr int E = D / 32;
-  const int heads = Hq + 2 * Hkv;
+  const int heads = p.Hq + 2 * p.Hkv;
   const long long wid = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
   if (wid >= T * heads) return;
   const int lane = threadIdx.x & 31;
   const long long t = wid / heads;
   const int h = static_cast<int>(wid - t * heads);
-  const __nv_bfloat16* src = qkv + (t * heads + h) * D;
+  const bool is_q = h < p.Hq;
+  const bool is_k = !is_q && h < p.Hq + p.Hkv;
+  const int hh = is_k ? h - p.Hq : h - p.Hq - p.Hkv;
+  const __nv_bfloat16* src = is_q ? p.q + t * p.q_ts + static_cast<long long>(h) * p.q_hs
+                                  : (is_k ? p.k + t * p.k_ts : p.v + t * p.v_ts) + static_cast<long long>(hh) * D;
   float v[E];
 #pragma unroll
   for (int j = 0; j < E; ++j) v[j] = __bfloat162float(src[lane + 32 * j]);
-  const bool is_q = h < Hq;
-  const bool is_k = !is_q && h < Hq + Hkv;
   if (is_q || is_k) {
-    const __nv_bfloat16* nw = is_q ? q_w : k_w;
+    const __nv_bfloat16* nw = is_q ? p.q_w : p.k_w;
     if (nw != nullptr) {
       float ss = 0.f;
 #pragma unroll
       for (int j = 0; j < E; ++j) ss += v[j] * v[j];
       ss = warp_sum(ss);
-      const float inv = rsqrtf(ss / D + eps);
+      const float inv = rsqrtf(ss / D + p.eps);
 #pragma unroll
       for (int j = 0; j < E; ++j) {
         // round to bf16 like the unfused norm would before the rotation
-        v[j] = __bfloat162float(__float2bfloat16(v[j] * inv * __bfloat162float(nw[lane + 32 * j])));
+        v[j] = __bfloat162float(__float2bfloat16(v[j] * inv * (__bfloat162float(nw[lane + 32 * j]) + p.w_add)));
       }
     }
-    if (cos_sin != nullptr) {
-      const float* cs = cos_sin + static_cast<long long>(positions[t]) * rd;
-      const int half = rd >> 1;
-      if (is_neox) {
-        constexpr int kMaxPairs = E / 2 > 0 ? E / 2 : 1;
-        const int pj = half / 32;            // register distance between partners
+    const float* cs = p.cos_sin + static_cast<long long>(p.positions[t]) * p.rd;
+    const int half = p.rd >> 1;
+    // pairs (2i, 2i + 1): the partner sits in the neighbouring lane
 #pragma unroll
-        for (int j = 0; j < kMaxPairs; ++j) {
-          if (j < pj) {
-            const int i = lane + 32 * j;     // index in the first half
-            const float c = cs[i], s = cs[half + i];
-            const float a = v[j], b = v[j + pj];
-            v[j] = a * c - b * s;
-            v[j + pj] = b * c + a * s;
-          }
-        }
-      } else {
-        // interleaved pairs (2p, 2p+1): partner sits in the neighbouring lane
-#pragma unroll
-        for (int j = 0; j < E; ++j) {
-          const int i = lane + 32 * j;
-          const float other = __shfl_xor_sync(0xffffffffu, v[j], 1);
-          if (i < rd) {
-            const int pidx = i >> 1;
-            const float c = cs[pidx], s = cs[half + pidx];
-            v[j] = (i & 1) ? (v[j] * c + other * s) : (v[j] * c - other * s);
-          }
-        }
+    for (int j = 0; j < E; ++j) {
+      const int i = lane + 32 * j;
+      const float other = __shfl_xor_sync(0xffffffffu, v[j], 1);
+      if (i < p.rd) {
+        const float c = cs[i >> 1], s = cs[half + (i >> 1)];
+        v[j] = (i & 1) ? (v[j] * c + other * s) : (v[j] * c - other * s);
       }
     }
   }
   __nv_bfloat16* dst;
   if (is_q) {
-    dst = q_out + (t * Hq + h) * D;
+    dst = p.q_out + (t * p.Hq + h) * D;
   } else {
-    if (kv == nullptr) return;
-    const int slot = loc[t];
-    const int page = slot / page_size, off = slot - page * page_size;
+    if (p.kv == nullptr) return;
+    const int slot = p.loc[t];
+    const int page = slot / p.page_size, off = slot - page * p.page_size;
 #ifdef SGLB_BOUNDS_CHECK
     if (g_dbg_kv_pages > 0 && (slot < 0 || page >= g_dbg_kv_pages)) {
       if (lane == 0) report(g_dbg_status, kOutOfBounds, static_cast<int>(t), slot);
       return;
     }
 #endif
-    const int kvsel = is_k ? 0 : 1;
-    const int hh = is_k ? h - Hq : h - Hq - Hkv;
-    dst = kv + ((((static_cast<long long>(page) * 2 + kvsel) * Hkv + hh) * page_size) + off) * D;
+    if (slot < 0) return;
+    dst = p.kv + ((((static_cast<long long>(page) * 2 + (is_k ? 0 : 1)) * p.Hkv + hh) * p.page_size) + off) * D;
   }
 #pragma unroll
   for (int j = 0; j < E; ++j) dst[lane + 32 * j] = __float2bfloat16(v[j]);
+}
+
+template <int D>
+cudaError_t launch_rope(const RopeParams& p, long long T, bool pairs, cudaStream_t s) {
+  const int heads = p.Hq + 2 * p.Hkv;
+  if (pairs) {
+    const long long blocks = (T * heads * 32 + 127) / 128;
+    return launch_pdl(rope_pairs_kernel<D>, dim3(blocks), dim3(128), 0, s, p, T);
+  }
+  // few tokens: a token's heads go to several CTAs, until there are a few for every SM
+  const int shares = (heads + kRopeThreads / (D / 8) - 1) / (kRopeThreads / (D / 8));
+  const long long want = (4ll * sm_count() + T - 1) / T;
+  return launch_pdl(rope_qknorm_kvwrite_kernel<D>, dim3(static_cast<unsigned>(T), static_cast<unsigned>(want < shares ? want : shares)),
+                    dim3(kRopeThreads), 0, s, p);
 }
 
 // page_table[rows[i], pos[i]] = ids[i]
@@ -425,37 +519,49 @@ int sglb_debug_set_kv_pages(int pages) {
 #endif
 }
 
-int sglb_rope_qknorm_kvwrite(void* q_out, const void* qkv, const int* positions, const float* cos_sin, const void* q_w,
-                             const void* k_w, float eps, long long T, int Hq, int Hkv, int D, int rotary_dim,
-                             void* kv_buffer, const int* loc, int page_size, int is_neox, cudaStream_t s) {
+// q: head h of token t at q + t * q_ts + h * q_hs; k, v: at k + t * k_ts + h * D, v + t * v_ts + h * D (all 16-byte units).  q_out
+// [T, Hq, D]; kv_buffer [pages, 2, Hkv, page_size, D] or null, loc the slots (< 0: not written).  Norm weights [D] (+ w_add) or null.
+// cos_sin fp32 [positions, rotary_dim] or null; is_neox: lane i turns with lane i + rotary_dim / 2 (rotary_dim a multiple of 16), else
+// neighbours turn.
+int sglb_rope_qknorm_kvwrite(void* q_out, const void* q, long long q_ts, int q_hs, const void* k, long long k_ts, const void* v,
+                             long long v_ts, const int* positions, const float* cos_sin, const void* q_w, const void* k_w, float w_add,
+                             float eps, long long T, int Hq, int Hkv, int D, int rotary_dim, void* kv_buffer, const int* loc,
+                             int page_size, int is_neox, cudaStream_t s) {
   using namespace sglb;
   if (T <= 0) return 0;
-  if (is_neox && cos_sin != nullptr && ((rotary_dim / 2) % 32 != 0 || rotary_dim > D)) return -kBadArgument;
-  const long long warps = T * (Hq + 2 * Hkv);
-  const int threads = 128;
-  const long long blocks = (warps * 32 + threads - 1) / threads;
-  auto* qo = static_cast<__nv_bfloat16*>(q_out);
-  auto* in = static_cast<const __nv_bfloat16*>(qkv);
-  auto* qw = static_cast<const __nv_bfloat16*>(q_w);
-  auto* kw = static_cast<const __nv_bfloat16*>(k_w);
-  auto* kv = static_cast<__nv_bfloat16*>(kv_buffer);
+  auto off = [](const void* a) { return reinterpret_cast<uintptr_t>(a) % 16 != 0; };
+  if (off(q) || off(k) || off(v) || off(q_out) || off(kv_buffer) || off(q_w) || off(k_w) || off(cos_sin) || q_ts % 8 || q_hs % 8 ||
+      k_ts % 8 || v_ts % 8 || T > 0x7fffffffll)
+    return -kBadArgument;
+  if (cos_sin != nullptr && (rotary_dim > D || rotary_dim % (is_neox ? 16 : 2) != 0)) return -kBadArgument;
+  RopeParams p{};
+  p.q_out = static_cast<__nv_bfloat16*>(q_out);
+  p.q = static_cast<const __nv_bfloat16*>(q);
+  p.k = static_cast<const __nv_bfloat16*>(k);
+  p.v = static_cast<const __nv_bfloat16*>(v);
+  p.q_ts = q_ts;
+  p.k_ts = k_ts;
+  p.v_ts = v_ts;
+  p.q_hs = q_hs;
+  p.positions = positions;
+  p.cos_sin = cos_sin;
+  p.q_w = static_cast<const __nv_bfloat16*>(q_w);
+  p.k_w = static_cast<const __nv_bfloat16*>(k_w);
+  p.w_add = w_add;
+  p.eps = eps;
+  p.Hq = Hq;
+  p.Hkv = Hkv;
+  p.rd = cos_sin != nullptr ? rotary_dim : 0;
+  p.kv = static_cast<__nv_bfloat16*>(kv_buffer);
+  p.loc = loc;
+  p.page_size = page_size;
+  const bool pairs = !is_neox && cos_sin != nullptr;
   switch (D) {
-    case 64:
-      launch_pdl(rope_qknorm_kvwrite_kernel<64>, dim3(blocks), dim3(threads), 0, s, qo, in, positions, cos_sin, qw, kw, eps, T, Hq, Hkv,
-                                                                rotary_dim, kv, loc, page_size, is_neox);
-      break;
-    case 128:
-      launch_pdl(rope_qknorm_kvwrite_kernel<128>, dim3(blocks), dim3(threads), 0, s, qo, in, positions, cos_sin, qw, kw, eps, T, Hq, Hkv,
-                                                                 rotary_dim, kv, loc, page_size, is_neox);
-      break;
-    case 256:
-      launch_pdl(rope_qknorm_kvwrite_kernel<256>, dim3(blocks), dim3(threads), 0, s, qo, in, positions, cos_sin, qw, kw, eps, T, Hq, Hkv,
-                                                                 rotary_dim, kv, loc, page_size, is_neox);
-      break;
-    default:
-      return -kBadArgument;
+    case 64: return static_cast<int>(launch_rope<64>(p, T, pairs, s));
+    case 128: return static_cast<int>(launch_rope<128>(p, T, pairs, s));
+    case 256: return static_cast<int>(launch_rope<256>(p, T, pairs, s));
+    default: return -kBadArgument;
   }
-  return static_cast<int>(cudaGetLastError());
 }
 
 int sglb_page_table_scatter(int* table, int max_pages, const int* rows, const int* pos, const int* ids, int n,

@@ -30,8 +30,10 @@ class RadixAttention(nn.Module):
         self.sliding_window_size = sliding_window_size or 0
         self.logit_cap = logit_cap or 0.0
 
-    def forward(self, qkv: torch.Tensor, forward_batch, rotary_emb=None, q_norm=None, k_norm=None,
+    def forward(self, qkv, forward_batch, rotary_emb=None, q_norm=None, k_norm=None,
                 sinks: torch.Tensor | None = None, gemma_norm: bool = False) -> torch.Tensor:
+        """`qkv [T, (heads + 2 kv_heads) * head_dim]`, or its three parts, `[T, heads of the part, head_dim]` each, which may be
+        strided."""
         fb = forward_batch
         pool = fb.token_to_kv_pool
         kv_buffer = pool.get_kv_buffer(self.layer_id)
@@ -42,6 +44,16 @@ class RadixAttention(nn.Module):
         rope = ops.rope_qknorm_kvwrite if not native_backend else reference.rope_qknorm_kvwrite
         attn = ops.paged_attention if not native_backend else reference.paged_attention
         eps = q_norm.variance_epsilon if q_norm is not None else 1e-6
+        rope_args = (rotary_emb.is_neox_style if rotary_emb is not None else True,
+                     rotary_emb.rotary_dim if rotary_emb is not None else None)
+        parts = None
+        if isinstance(qkv, tuple):
+            parts, qkv = qkv, None
+            tensors = (fb.positions, rotary_emb.cos_sin_cache if rotary_emb is not None else None,
+                       q_norm.weight if q_norm is not None else None, k_norm.weight if k_norm is not None else None)
+            if native_backend or hasattr(rotary_emb, "mrope_section") \
+                    or not ops.rope_parts_supported(*parts, *tensors, kv_buffer, loc, *rope_args):
+                qkv, parts = torch.cat([t.flatten(1) for t in parts], dim=-1), None
         mpos = fb.extras.get("mrope_positions") if hasattr(rotary_emb, "mrope_section") else None
         if mpos is not None:
             # multimodal rotary: the frequency lanes are driven by three position streams, so the
@@ -54,14 +66,15 @@ class RadixAttention(nn.Module):
                 q_norm = k_norm = None
             q3, k3 = rotary_emb(mpos, q3, k3)
             qkv = torch.cat([q3.flatten(1), k3.flatten(1), qkv[:, qs + ks:]], dim=-1)
-            rotary_emb = None
-        q = rope(qkv, fb.positions,
-                 rotary_emb.cos_sin_cache if rotary_emb is not None else None,
-                 q_norm.weight if q_norm is not None else None,
-                 k_norm.weight if k_norm is not None else None,
-                 eps, self.num_heads, self.num_kv_heads, self.head_dim, kv_buffer, loc, fb.page_size,
-                 rotary_emb.is_neox_style if rotary_emb is not None else True,
-                 rotary_emb.rotary_dim if rotary_emb is not None else None, gemma_norm)
+            rotary_emb, rope_args = None, (True, None)
+        if parts is not None:
+            q = ops.rope_parts(*parts, *tensors, eps, kv_buffer, loc, fb.page_size, *rope_args, gemma_norm)
+        else:
+            q = rope(qkv, fb.positions,
+                     rotary_emb.cos_sin_cache if rotary_emb is not None else None,
+                     q_norm.weight if q_norm is not None else None,
+                     k_norm.weight if k_norm is not None else None,
+                     eps, self.num_heads, self.num_kv_heads, self.head_dim, kv_buffer, loc, fb.page_size, *rope_args, gemma_norm)
         page_table = fb.page_table
         if hasattr(pool, "is_swa_layer") and pool.is_swa_layer(self.layer_id):
             page_table = fb.extras["swa_page_table"]

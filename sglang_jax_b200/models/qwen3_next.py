@@ -9,6 +9,7 @@ from __future__ import annotations
 import torch
 from torch import nn
 
+from .. import ops
 from ..layers.embeddings import ParallelLMHead, VocabParallelEmbedding, get_rope
 from ..layers.layernorm import GemmaRMSNorm
 from ..layers.linear import ColumnParallelLinear, RowParallelLinear
@@ -48,11 +49,12 @@ class GatedAttention(nn.Module):
     def forward(self, x, fb):
         T = x.shape[0]
         qg = self.q_proj(x).view(T, self.nh, 2 * self.head_dim)
-        q, gate = qg[..., : self.head_dim], qg[..., self.head_dim:]
-        qkv = torch.cat([q.reshape(T, -1), self.k_proj(x), self.v_proj(x)], dim=-1)
-        o = self.attn(qkv, fb, self.rotary_emb, self.q_norm, self.k_norm, gemma_norm=True)
-        o = o * torch.sigmoid(gate.reshape(T, -1).float()).to(o.dtype)
-        return self.o_proj(o)
+        q = qg[..., : self.head_dim]
+        k, v = (y.view(T, self.nkv, self.head_dim) for y in (self.k_proj(x), self.v_proj(x)))
+        o = self.attn((q, k, v), fb, self.rotary_emb, self.q_norm, self.k_norm, gemma_norm=True)
+        # a row per token and head: the gate's rows lie two heads apart in the projection
+        o = ops.sigmoid_gate(o.reshape(T * self.nh, self.head_dim), qg.view(T * self.nh, 2 * self.head_dim)[:, self.head_dim:])
+        return self.o_proj(o.view(T, self.nh * self.head_dim))
 
 
 class Qwen3NextDecoderLayer(nn.Module):

@@ -326,16 +326,42 @@ def linear(x, w, bias=None):
     return reference.linear(x, w, bias)
 
 
+def linear_swiglu_supported(x, w) -> bool:
+    """Whether `linear_swiglu` computes `silu_and_mul(linear(x, w))` for these operands: prefill sizes, whole blocks of K, and no fused
+    all-gather that somebody has to wait for."""
+    if not (use_native(x) and w.dtype == torch.bfloat16 and x.dim() == 2 and w.is_contiguous() and x.stride(1) == 1):
+        return False
+    from ..parallel import state as ps
+    comm = ps.get_state().fused_comm
+    return (x.shape[0] > 256 and x.shape[1] % 64 == 0 and w.shape[0] % 16 == 0 and x.stride(0) % 8 == 0 and x.stride(0) >= x.shape[1]
+            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and (comm is None or comm.pending_gather is None))
+
+
+def linear_swiglu(x, w):
+    """`silu(gate) * up`, gate and up the halves of `x w^T`, from the fp32 sums (no rounding in between)."""
+    return _native().gemm_pair(x, w, gated=True)
+
+
 def rope_qknorm_kvwrite(qkv, positions, cos_sin, q_norm_w, k_norm_w, eps, num_q_heads, num_kv_heads,
                         head_dim, kv_buffer, out_cache_loc, page_size, is_neox=True, rotary_dim=None,
                         gemma_norm=False):
-    if use_native(qkv) and (kv_buffer is None or kv_buffer.dtype == torch.bfloat16) and not gemma_norm:
+    if use_native(qkv) and (kv_buffer is None or kv_buffer.dtype == torch.bfloat16):
         return _native().rope_qknorm_kvwrite(qkv, positions, cos_sin, q_norm_w, k_norm_w, eps, num_q_heads,
                                              num_kv_heads, head_dim, kv_buffer, out_cache_loc, page_size,
-                                             is_neox, rotary_dim)
+                                             is_neox, rotary_dim, gemma_norm)
     return reference.rope_qknorm_kvwrite(qkv, positions, cos_sin, q_norm_w, k_norm_w, eps, num_q_heads,
                                          num_kv_heads, head_dim, kv_buffer, out_cache_loc, page_size,
                                          is_neox, rotary_dim, gemma_norm)
+
+
+def rope_parts_supported(q, k, v, positions, cos_sin, q_norm_w, k_norm_w, kv_buffer, *a) -> bool:
+    """Whether queries, keys and values that lie apart need not be concatenated for `rope_qknorm_kvwrite`."""
+    return use_native(q) and kv_buffer.dtype == torch.bfloat16 and \
+        _native().rope_parts_supported(q, k, v, positions, cos_sin, q_norm_w, k_norm_w, kv_buffer, *a)
+
+
+def rope_parts(*a):
+    return _native().rope_parts(*a)
 
 
 def paged_attention(q, kv_buffer, page_table, req_pool_indices, seq_lens, page_size, scale,

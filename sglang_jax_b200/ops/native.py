@@ -71,9 +71,8 @@ def lib():
     sig("sglb_silu_and_mul", [c_void_p, c_void_p, c_longlong, c_int, c_void_p])
     sig("sglb_embedding", [c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p])
     sig("sglb_argmax", [c_void_p, c_void_p, c_int, c_int, c_longlong, c_int, c_void_p])
-    sig("sglb_rope_qknorm_kvwrite", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float,
-                                           c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int,
-                                           c_void_p])
+    sig("sglb_rope_qknorm_kvwrite", [c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_void_p, c_longlong]
+        + [c_void_p] * 4 + [c_float, c_float, c_longlong] + [c_int] * 4 + [c_void_p, c_void_p, c_int, c_int, c_void_p])
     sig("sglb_page_table_scatter", [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p])
     sig("sglb_resolve_future", [c_void_p, c_void_p, c_int, c_void_p])
     sig("sglb_decode_num_splits", [c_int, c_int, c_int])
@@ -352,22 +351,50 @@ def linear_part(x, w):
     return out
 
 
+def rope_parts_supported(q, k, v, positions, cos_sin, q_norm_w, k_norm_w, kv_buffer, loc, is_neox, rotary_dim) -> bool:
+    """Whether `rope_parts` takes these tensors: `q [T, Hq, D]`, `k`, `v [T, Hkv, D]`."""
+    D = q.shape[2]
+    rd = rotary_dim or D
+    step = cos_sin is None or (rd % 16 == 0 if is_neox else rd % 2 == 0)
+    norms = [w for w in (q_norm_w, k_norm_w) if w is not None]
+    heads = all(t.stride(2) == 1 and (t.shape[1] == 1 or t.stride(1) == D) for t in (k, v)) and q.stride(2) == 1
+    aligned = all(t.data_ptr() % 16 == 0 and t.stride(0) % 8 == 0 for t in (q, k, v)) and q.stride(1) % 8 == 0
+    return (D in (64, 128, 256) and step and rd <= D and heads and aligned and positions.dtype == torch.int32
+            and all(t.dtype == torch.bfloat16 for t in (q, k, v, *norms)) and all(w.data_ptr() % 16 == 0 for w in norms)
+            and (cos_sin is None or (cos_sin.dtype == torch.float32 and cos_sin.data_ptr() % 16 == 0))
+            and (kv_buffer is None or (kv_buffer.data_ptr() % 16 == 0 and kv_buffer.is_contiguous() and loc.dtype == torch.int32)))
+
+
+def rope_parts(q, k, v, positions, cos_sin, q_norm_w, k_norm_w, eps, kv_buffer, loc, page_size, is_neox=True, rotary_dim=None,
+               gemma_norm=False):
+    """`rope_qknorm_kvwrite` of queries, keys and values that lie apart (`q [T, Hq, D]`, `k`, `v [T, Hkv, D]` by strides)."""
+    T, Hq, D = q.shape
+    out = torch.empty((T, Hq, D), dtype=q.dtype, device=q.device)
+    _check(lib().sglb_rope_qknorm_kvwrite(_p(out), q.data_ptr(), q.stride(0), q.stride(1), k.data_ptr(), k.stride(0), v.data_ptr(),
+                                          v.stride(0), _p(positions), _p(cos_sin), _p(q_norm_w), _p(k_norm_w),
+                                          1.0 if gemma_norm else 0.0, eps, T, Hq, k.shape[1], D, rotary_dim or D, _p(kv_buffer), _p(loc),
+                                          page_size, int(is_neox), _stream()), "rope_qknorm_kvwrite")
+    return out
+
+
 def rope_qknorm_kvwrite(qkv, positions, cos_sin, q_norm_w, k_norm_w, eps, num_q_heads, num_kv_heads, head_dim,
-                        kv_buffer, out_cache_loc, page_size, is_neox=True, rotary_dim=None):
+                        kv_buffer, out_cache_loc, page_size, is_neox=True, rotary_dim=None, gemma_norm=False):
     qkv = qkv.contiguous()
-    T = qkv.shape[0]
-    rd = rotary_dim or head_dim
-    if (is_neox and cos_sin is not None and (rd // 2) % 32 != 0) or head_dim not in (64, 128, 256) \
-            or positions.dtype != torch.int32 or (out_cache_loc is not None and out_cache_loc.dtype != torch.int32):
+    T, qs, ks = qkv.shape[0], num_q_heads * head_dim, num_kv_heads * head_dim
+    rd, ld, at = rotary_dim or head_dim, qs + 2 * ks, qkv.data_ptr()
+    if head_dim not in (64, 128, 256) or qkv.shape[1] != ld or at % 16 or positions.dtype != torch.int32 \
+            or (cos_sin is not None and (rd % (16 if is_neox else 2) or rd > head_dim)) \
+            or (kv_buffer is not None and out_cache_loc.dtype != torch.int32) \
+            or any(w is not None and (w.dtype != torch.bfloat16 or w.data_ptr() % 16) for w in (q_norm_w, k_norm_w)):
         from . import reference
         return reference.rope_qknorm_kvwrite(qkv, positions, cos_sin, q_norm_w, k_norm_w, eps, num_q_heads,
                                              num_kv_heads, head_dim, kv_buffer, out_cache_loc, page_size, is_neox,
-                                             rotary_dim)
+                                             rotary_dim, gemma_norm)
     q = torch.empty((T, num_q_heads, head_dim), dtype=qkv.dtype, device=qkv.device)
-    _check(lib().sglb_rope_qknorm_kvwrite(_p(q), _p(qkv), _p(positions), _p(cos_sin), _p(q_norm_w), _p(k_norm_w),
-                                          eps, T, num_q_heads, num_kv_heads, head_dim, rd, _p(kv_buffer),
-                                          _p(out_cache_loc), page_size, int(is_neox), _stream()),
-           "rope_qknorm_kvwrite")
+    _check(lib().sglb_rope_qknorm_kvwrite(q.data_ptr(), at, ld, head_dim, at + 2 * qs, ld, at + 2 * (qs + ks), ld, _p(positions),
+                                          _p(cos_sin), _p(q_norm_w), _p(k_norm_w), 1.0 if gemma_norm else 0.0, eps, T, num_q_heads,
+                                          num_kv_heads, head_dim, rd, _p(kv_buffer), _p(out_cache_loc), page_size, int(is_neox),
+                                          _stream()), "rope_qknorm_kvwrite")
     return q
 
 

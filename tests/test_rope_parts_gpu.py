@@ -1,0 +1,51 @@
+"""Norm, rotation and cache write of queries, keys and values, and the fused gated product, on the GPU."""
+
+import pytest
+import torch
+
+from sglang_jax_b200 import ops
+from sglang_jax_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("T,Hq,Hkv,D", [(1, 16, 4, 128), (3, 1, 1, 64), (300, 5, 2, 128), (37, 3, 1, 256), (700, 64, 8, 128)])
+@pytest.mark.parametrize("rd,neox", [(1.0, True), (0.5, True), (0.25, True), (1.0, False), (0.5, False), (0.0, True)])
+@pytest.mark.parametrize("norm,gemma", [(False, False), (True, False), (True, True)])
+def test_rope_parts(T, Hq, Hkv, D, rd, neox, norm, gemma):
+    torch.manual_seed(T + D)
+    dev, bf, P = "cuda", torch.bfloat16, 16
+    rd = int(D * rd)
+    qg = torch.randn(T, Hq, 2 * D, device=dev, dtype=bf)                      # a gate behind every query
+    q, k, v = qg[..., :D], torch.randn(T, Hkv, D, device=dev, dtype=bf), torch.randn(T, Hkv, D, device=dev, dtype=bf)
+    pos = torch.randint(0, 500, (T,), device=dev, dtype=torch.int32)
+    cs = ref.build_cos_sin_cache(rd, 500, 1e4, device=dev) if rd else None
+    qw, kw = ((torch.randn(D, device=dev, dtype=bf) * 0.2 + (0.0 if gemma else 1.0)) if norm else None for _ in range(2))
+    loc = torch.randperm(T + 40, device=dev)[:T].int()
+    cache = torch.zeros((T + 40) // P + 1, 2, Hkv, P, D, device=dev, dtype=bf)
+    got_kv, want_kv, fused_kv = cache.clone(), cache.clone(), cache.clone()
+    qkv = torch.cat([q.flatten(1), k.flatten(1), v.flatten(1)], -1)
+    want = ref.rope_qknorm_kvwrite(qkv, pos, cs, qw, kw, 1e-6, Hq, Hkv, D, want_kv, loc, P, neox, rd or None, gemma)
+    args = (pos, cs, qw, kw)
+    assert ops.rope_parts_supported(q, k, v, *args, got_kv, loc, neox, rd or None)
+    got = ops.rope_parts(q, k, v, *args, 1e-6, got_kv, loc, P, neox, rd or None, gemma)
+    fused = ops.rope_qknorm_kvwrite(qkv, *args, 1e-6, Hq, Hkv, D, fused_kv, loc, P, neox, rd or None, gemma)
+    assert torch.equal(fused, got) and torch.equal(fused_kv, got_kv)
+    # the norm's rounding to bf16 may fall the other way (2^-8 of a value at most); a rotation adds two such values and rounds again
+    for a, b in ((got, want), (got_kv, want_kv)):
+        assert (a.float() - b.float()).abs().max() <= 2 ** -6 * max(b.float().abs().max().item(), 1.0)
+        assert (a.float() - b.float()).norm() <= 2e-3 * b.float().norm()
+    assert torch.equal(got_kv[:, 1], want_kv[:, 1])
+
+
+@pytest.mark.parametrize("T,K,I", [(257, 64, 8), (300, 192, 136), (1000, 2048, 768)])
+def test_linear_swiglu(T, K, I):
+    torch.manual_seed(T)
+    x = torch.randn(T, K, device="cuda", dtype=torch.bfloat16)
+    w = torch.randn(2 * I, K, device="cuda", dtype=torch.bfloat16) * K ** -0.5
+    assert ops.linear_swiglu_supported(x, w) and not ops.linear_swiglu_supported(x[:256], w)
+    h = x.double() @ w.double().t()
+    want = torch.nn.functional.silu(h[:, :I]) * h[:, I:]
+    err = lambda y: ((y.double() - want).norm() / want.norm()).item()
+    assert err(ops.linear_swiglu(x, w)) < 2 ** -8                             # one rounding to bf16
+    assert err(ops.linear_swiglu(x, w)) <= err(ops.silu_and_mul(ops.linear(x, w)))
