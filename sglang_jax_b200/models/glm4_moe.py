@@ -35,7 +35,7 @@ class Glm4MoeDecoderLayer(nn.Module):
         if self.is_sparse:
             return partial_add_norm(lambda out: self.mlp.partial(h, out), h.shape[0], h.shape[1], residual, next_norm,
                                     self.mlp.tp_size, block=self.mlp, x=h)
-        act = self.mlp.act_fn(self.mlp.gate_up_proj(h))
+        act = self.mlp.activated(h)
         return row_linear_add_norm(self.mlp.down_proj, act, residual, next_norm)
 
 

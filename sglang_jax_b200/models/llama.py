@@ -14,6 +14,7 @@ from typing import Iterable
 import torch
 from torch import nn
 
+from .. import ops
 from ..layers.activation import SiluAndMul
 from ..layers.embeddings import ParallelLMHead, VocabParallelEmbedding, get_rope
 from ..layers.fused_block import row_linear_add_norm
@@ -31,8 +32,17 @@ class DenseMLP(nn.Module):
         self.down_proj = RowParallelLinear(intermediate_size, hidden_size, bias, dtype, reduce_results=True)
         self.act_fn = SiluAndMul()
 
+    def activated(self, x):
+        """`act_fn(gate_up_proj(x))`, in one kernel where that is a plain product of prefill size."""
+        up = self.gate_up_proj
+        plain = up.qweight is None and up.lora is None and up.bias is None and type(self.act_fn) is SiluAndMul \
+            and not (up._forward_hooks or up._forward_pre_hooks or self.act_fn._forward_hooks or self.act_fn._forward_pre_hooks)
+        if plain and ops.linear_swiglu_supported(x, up.weight):
+            return ops.linear_swiglu(x, up.weight)
+        return self.act_fn(up(x))
+
     def forward(self, x):
-        return self.down_proj(self.act_fn(self.gate_up_proj(x)))
+        return self.down_proj(self.activated(x))
 
 
 class UngatedMLP(nn.Module):
@@ -98,7 +108,7 @@ class DenseDecoderLayer(nn.Module):
         attn_out = self.self_attn(hidden_normed, forward_batch)
         h, residual = row_linear_add_norm(self.self_attn.o_proj, attn_out, residual,
                                           self.post_attention_layernorm, consumer=self.mlp.gate_up_proj)
-        act = self.mlp.act_fn(self.mlp.gate_up_proj(h))
+        act = self.mlp.activated(h)
         return row_linear_add_norm(self.mlp.down_proj, act, residual, next_norm, consumer=next_consumer)
 
 
