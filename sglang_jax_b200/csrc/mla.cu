@@ -349,24 +349,46 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
   }
 }
 
-__global__ void mla_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse,
-                                   __nv_bfloat16* __restrict__ out, int num_splits, int R, int H, const ScoreTerms terms) {
-  const int row = blockIdx.x;   // b * H + h
-  const float* lse = part_lse + static_cast<size_t>(row) * num_splits;
-  float mmax = -INFINITY;
-  for (int s = 0; s < num_splits; ++s) mmax = fmaxf(mmax, lse[s]);
-  const float sink = terms.sink_log2(row % H);
-  mmax = fmaxf(mmax, sink);
-  float wsum = sink == -INFINITY ? 0.f : exp2f(sink - mmax);
-  for (int s = 0; s < num_splits; ++s) wsum += (lse[s] == -INFINITY) ? 0.f : exp2f(lse[s] - mmax);
-  const float inv = wsum > 0.f ? 1.f / wsum : 0.f;
-  for (int d = threadIdx.x; d < R; d += blockDim.x) {
-    float acc = 0.f;
-    for (int s = 0; s < num_splits; ++s) {
-      const float w = (lse[s] == -INFINITY) ? 0.f : exp2f(lse[s] - mmax);
-      acc += w * part_o[(static_cast<size_t>(row) * num_splits + s) * R + d];
+// One CTA per (query, head).  The weights of the splits are computed once, by a warp, and the partial rows come eight at a time, all
+// in flight together (one after another, each with an exponential of its own: 20 us for 7 queries of 16 heads in 32 splits).
+__global__ void __launch_bounds__(128)
+mla_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse,
+                   __nv_bfloat16* __restrict__ out, int num_splits, int R, int H, const ScoreTerms terms) {
+  extern __shared__ float weight[];                      // [num_splits]
+  const int row = blockIdx.x, lane = threadIdx.x & 31;   // row = b * H + h
+  pdl_wait();
+  if (threadIdx.x < 32) {
+    const float* lse = part_lse + static_cast<size_t>(row) * num_splits;
+    const float sink = terms.sink_log2(row % H);
+    float top = sink, sum = 0.f;
+    for (int s = lane; s < num_splits; s += 32) top = fmaxf(top, lse[s]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    for (int s = lane; s < num_splits; s += 32) {
+      const float w = lse[s] == -INFINITY ? 0.f : exp2f(lse[s] - top);
+      weight[s] = w;
+      sum += w;
     }
-    out[static_cast<size_t>(row) * R + d] = __float2bfloat16(acc * inv);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    sum += sink == -INFINITY ? 0.f : exp2f(sink - top);
+    for (int s = lane; s < num_splits; s += 32) weight[s] = sum > 0.f ? weight[s] / sum : 0.f;
+  }
+  __syncthreads();
+  const float* part = part_o + static_cast<size_t>(row) * num_splits * R;
+  for (int d = threadIdx.x; d < R; d += 128) {
+    float acc = 0.f;
+    for (int s0 = 0; s0 < num_splits; s0 += 8) {
+      float v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = s0 + i < num_splits ? part[static_cast<size_t>(s0 + i) * R + d] : 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float w = s0 + i < num_splits ? weight[s0 + i] : 0.f;
+        if (w != 0.f) acc += w * v[i];        // (a split without a key may hold anything)
+      }
+    }
+    out[static_cast<size_t>(row) * R + d] = __float2bfloat16(acc);
   }
 }
 
@@ -451,7 +473,7 @@ int sglb_mla_decode(const void* q_lat, const void* q_pe, long long pe_token_stri
   const int dk = kv_lora_rank + rope_dim;
   if (kv_lora_rank < 1 || kv_lora_rank > 512 || rope_dim < 1 || dk > row_elems || row_elems % 8 != 0) return -kBadArgument;
   if (page_size < TN ? (TN % page_size != 0) : (page_size % TN != 0)) return -kBadArgument;
-  if (num_splits > 1 && (part_o == nullptr || part_lse == nullptr)) return -kBadArgument;
+  if (num_splits > 1 && (part_o == nullptr || part_lse == nullptr || num_splits > 4096)) return -kBadArgument;
   MlaParams p{};
   // one block past the key when the output lanes of the widest warp group reach further (they are not stored)
   const int ng = (kv_lora_rank + 63) / 64;
@@ -483,8 +505,8 @@ int sglb_mla_decode(const void* q_lat, const void* q_pe, long long pe_token_stri
   p.terms = ScoreTerms{0.f, nullptr, sink};
   cudaError_t e = exact ? launch_width<true>(tm, p, smem, stream) : launch_width<false>(tm, p, smem, stream);
   if (e == cudaSuccess && p.num_splits > 1) {
-    mla_combine_kernel<<<B * H, 128, 0, stream>>>(part_o, part_lse, p.out, p.num_splits, kv_lora_rank, H, p.terms);
-    e = cudaGetLastError();
+    e = launch_pdl(mla_combine_kernel, dim3(B * H), dim3(128), num_splits * sizeof(float), stream, part_o, part_lse, p.out, p.num_splits, kv_lora_rank, H,
+                   p.terms);
   }
   return e == cudaSuccess ? 0 : static_cast<int>(e);
 }

@@ -39,7 +39,7 @@ __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return _
 constexpr int kRouterWarps = 8;
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
@@ -61,25 +61,32 @@ router_logits_kernel(float* __restrict__ out, const __nv_bfloat16* __restrict__ 
 #pragma unroll
   for (int n = 0; n < NT; ++n) wb[n] = w + static_cast<size_t>(min(e0 + 8 * n + g, E - 1)) * K + 8 * t4;
   float sum[MT][NT][4] = {};
-#pragma unroll(MT == 1 ? 4 : 1)
-  for (int k = 32 * warp; k < K; k += 32 * kRouterWarps) {
-    uint4 a[MT][2], b[NT];
+  constexpr int kRuns = MT == 1 ? 4 : 1;                     // runs whose loads are in flight together
+  for (int k0 = 32 * warp; k0 < K; k0 += 32 * kRouterWarps * kRuns) {
+    uint4 a[kRuns][MT][2], b[kRuns][NT];
 #pragma unroll
-    for (int m = 0; m < MT; ++m)
+    for (int r = 0; r < kRuns; ++r) {
+      const int k = k0 + 32 * kRouterWarps * r;
+      const bool in = k < K;                                  // (zeros add nothing)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) a[m][h] = __ldg(reinterpret_cast<const uint4*>(xa[m][h] + k));
+      for (int m = 0; m < MT; ++m)
 #pragma unroll
-    for (int n = 0; n < NT; ++n) b[n] = __ldg(reinterpret_cast<const uint4*>(wb[n] + k));
+        for (int h = 0; h < 2; ++h) a[r][m][h] = in ? __ldg(reinterpret_cast<const uint4*>(xa[m][h] + k)) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-    for (int m = 0; m < MT; ++m)
+      for (int n = 0; n < NT; ++n) b[r][n] = in ? __ldg(reinterpret_cast<const uint4*>(wb[n] + k)) : make_uint4(0, 0, 0, 0);
+    }
 #pragma unroll
-      for (int n = 0; n < NT; ++n) {
-        float c[4] = {0.f, 0.f, 0.f, 0.f};
-        mma_bf16(c, a[m][0].x, a[m][1].x, a[m][0].y, a[m][1].y, b[n].x, b[n].y);
-        mma_bf16(c, a[m][0].z, a[m][1].z, a[m][0].w, a[m][1].w, b[n].z, b[n].w);
+    for (int r = 0; r < kRuns; ++r)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) sum[m][n][i] += c[i];
-      }
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+          float c[4] = {0.f, 0.f, 0.f, 0.f};
+          mma_bf16(c, a[r][m][0].x, a[r][m][1].x, a[r][m][0].y, a[r][m][1].y, b[r][n].x, b[r][n].y);
+          mma_bf16(c, a[r][m][0].z, a[r][m][1].z, a[r][m][0].w, a[r][m][1].w, b[r][n].z, b[r][n].w);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) sum[m][n][i] += c[i];
+        }
   }
 #pragma unroll
   for (int m = 0; m < MT; ++m)
