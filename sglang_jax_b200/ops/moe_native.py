@@ -111,10 +111,12 @@ def moe_gather(x, ws: MoeWorkspace, max_rows: int):
     return out
 
 
-def on_pairs(rows: int, K: int) -> bool:
+def on_pairs(rows: int, K: int, experts: int) -> bool:
     """Whether a grouped product of `rows` rows runs on pairs of SMs (`csrc/gemm_pair.cu`): its maps want whole blocks of 64 lanes.  Up
-    to 256 rows the weights' bytes are shared out evenly over all SMs instead."""
-    return rows > 256 and K % 64 == 0
+    to 256 rows the other kernel shares the bytes of all experts out evenly over all SMs, which is good while most of few experts are
+    chosen.  Both products of 768 x 2048, pairs against that, 64 experts: 37 / 66 us at 8 rows, 96 / 88 at 56, 125 / 118 at 128,
+    135 / 137 at 256; 128 experts: 117 / 134 at 64 rows, 206 / 232 at 256."""
+    return K % 64 == 0 and (rows > 256 or experts >= 128 or 2 * rows <= experts)
 
 
 def pair_tile(rows: int, experts: int) -> int:
@@ -143,7 +145,7 @@ def grouped_gemm_pair(x_sorted, w, ws: MoeWorkspace, rows: int, gated: bool = Fa
 def grouped_gemm(x_sorted, w, ws: MoeWorkspace, rows: int):
     """`x_sorted [rows, K]` (rows sorted by expert), `w [E_local, N, K]` -> `[rows, N]`."""
     E, N, K = w.shape
-    if on_pairs(rows, K):
+    if on_pairs(rows, K, E):
         return grouped_gemm_pair(x_sorted, w, ws, rows)
     assert ws.tile_rows == TILE_ROWS or rows <= 256
     out = torch.empty((rows, N), dtype=x_sorted.dtype, device=x_sorted.device)
@@ -253,7 +255,7 @@ def fused_experts(x, w13, w2, topk_weights, topk_ids, expert_start: int = 0, ws:
     pairs = T * k
     if ws is None or ws.max_pairs < pairs:
         ws = MoeWorkspace(pairs, E_local, x.device)
-    if on_pairs(pairs, H) and on_pairs(pairs, w2.shape[2]):
+    if on_pairs(pairs, H, E_local) and on_pairs(pairs, w2.shape[2], E_local):
         moe_align(topk_ids, expert_start, E_local, ws, tile_rows=pair_tile(pairs, E_local))
         a = grouped_gemm_pair(moe_gather(x, ws, pairs), w13, ws, pairs, gated=True)
     else:

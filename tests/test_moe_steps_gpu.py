@@ -71,7 +71,8 @@ def test_moe_combine(T, k, H, shared):
     torch.testing.assert_close(got.double(), want, rtol=2 ** -8, atol=1e-5)   # one rounding to bf16
 
 
-@pytest.mark.parametrize("T,k,E,H,I", [(300, 1, 3, 128, 64), (257, 8, 64, 256, 200), (1024, 8, 8, 192, 320), (33, 8, 64, 512, 128),
+@pytest.mark.parametrize("T,k,E,H,I", [(1, 8, 64, 256, 128), (8, 8, 128, 128, 64), (4, 8, 64, 64, 192), (20, 8, 64, 256, 128), (300, 1, 3, 128, 64),
+                                       (257, 8, 64, 256, 200), (1024, 8, 8, 192, 320), (33, 8, 64, 512, 128),
                                        (700, 2, 128, 64, 264)])
 def test_fused_experts(T, k, E, H, I):
     """Products on pairs of SMs (whole blocks of 64 lanes) and the general ones against fp32 arithmetic."""
