@@ -57,10 +57,12 @@ def topk_route(router_logits, top_k, scoring="softmax", renormalize=True, correc
 
 
 def router_logits_supported(x, weight, bias=None) -> bool:
-    return (x.dim() == 2 and x.dtype == weight.dtype == torch.bfloat16 and weight.is_contiguous() and x.shape[1] % 32 == 0
+    return (x.dim() == weight.dim() == 2 and x.dtype == weight.dtype == torch.bfloat16 and weight.is_contiguous()
+            and x.shape[1] == weight.shape[1] > 0 and x.shape[1] % 32 == 0 and weight.shape[0] > 0
             and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.stride(0) >= x.shape[1] and x.data_ptr() % 16 == 0
             and weight.data_ptr() % 16 == 0 and x.device == weight.device
-            and (bias is None or (bias.dtype == torch.bfloat16 and bias.is_contiguous())))
+            and (bias is None or (bias.dtype == torch.bfloat16 and bias.is_contiguous() and bias.shape == weight.shape[:1]
+                                  and bias.device == x.device)))
 
 
 def router_logits(x, weight, bias=None):
