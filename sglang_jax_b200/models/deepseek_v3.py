@@ -70,8 +70,9 @@ class MLAAttention(nn.Module):
         """Split kv_b_proj into the two per-head matrices of the absorbed form (after loading)."""
         w = self.kv_b_proj.weight.data.view(self.local_heads, self.nope + self.v_dim, self.kv_lora)
         self.w_up = w
-        self.w_uk = w[:, : self.nope, :].contiguous()
-        self.w_uv = w[:, self.nope:, :].transpose(1, 2).contiguous()
+        # (stored with the summed lanes innermost: the query's in a copy, the value's as the projection's own rows)
+        self.w_uk = w[:, : self.nope, :].transpose(1, 2).contiguous().transpose(1, 2)
+        self.w_uv = w[:, self.nope:, :].transpose(1, 2)
 
     def forward(self, x, fb):
         T = x.shape[0]
@@ -121,19 +122,10 @@ class MLAAttention(nn.Module):
 
     def _latent_query(self, q):
         """Absorbed query: `[T, h, nope] x [h, nope, r] -> [T, h, r]`."""
-        q_nope = q[..., : self.nope]
-        if not ops.use_native(q) or self.w_uk.dtype != q.dtype:
-            return torch.einsum("thn,hnr->thr", q_nope.float(), self.w_uk.float()).to(q.dtype)
-        out = torch.empty(q.shape[0], self.local_heads, self.kv_lora, dtype=q.dtype, device=q.device)
-        torch.bmm(q_nope.transpose(0, 1), self.w_uk, out=out.transpose(0, 1))
-        return out
+        return ops.head_product(q[..., : self.nope], self.w_uk)
 
     def _value_up(self, o_lat):
-        if not ops.use_native(o_lat) or self.w_uv.dtype != o_lat.dtype:
-            return torch.einsum("thr,hrv->thv", o_lat.float(), self.w_uv.float()).to(o_lat.dtype)
-        out = torch.empty(o_lat.shape[0], self.local_heads, self.v_dim, dtype=o_lat.dtype, device=o_lat.device)
-        torch.bmm(o_lat.transpose(0, 1), self.w_uv, out=out.transpose(0, 1))
-        return out
+        return ops.head_product(o_lat, self.w_uv)
 
     def _tiled(self, q, q_pe, buf, fb, allowed) -> bool:
         """Whether the sequences of an extend step can go through the prefill kernel (long ones: keys and values of what they see

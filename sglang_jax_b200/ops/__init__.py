@@ -261,6 +261,13 @@ def latent_prep(proj, *a, **kw):
     return (_native() if use_native_wide(proj) else reference).latent_prep(proj, *a, **kw)
 
 
+def head_product(x, w):
+    """`x [T, H, K]` times `w [H, K, N]` per head, summed in fp32 -> `[T, H, N]` in x's type."""
+    if use_native(x) and _native().head_product_supported(x, w):
+        return _native().head_product(x, w)
+    return reference.head_product(x, w)
+
+
 def mla_prep_supported(q, *a) -> bool:
     return use_native(q) and _native().mla_prep_supported(q, *a)
 

@@ -117,6 +117,7 @@ def lib():
                                                                     c_void_p])
     sig("sglb_mla_prep", [c_void_p, c_longlong, c_void_p, c_longlong] + [c_int] * 5 + [c_void_p, c_float, c_float, c_void_p, c_int,
                           c_void_p, c_void_p, c_void_p, c_int, c_void_p])
+    sig("sglb_head_product", [c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_longlong] + [c_int] * 5 + [c_void_p])
     sig("sglb_latent_rotate", [c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p])
     sig("sglb_latent_attn_any", [c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p,
                                  c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_int, c_void_p])
@@ -683,6 +684,25 @@ def mla_decode(q_latent, q_pe, kv_buffer, page_table, req_pool_indices, seq_lens
                                  _p(req_pool_indices), _p(seq_lens), B, H, R, q_pe.shape[-1], page_size, scale,
                                  int(window), _per_head(sink, H), num_splits, _p(part_o), _p(part_lse), int(exact), _stream()),
            "mla_decode")
+    return out
+
+
+# ---- per-head products around the absorbed latent attention (csrc/head_product.cu)
+def head_product_supported(x, w) -> bool:
+    """Whether `head_product` takes these operands."""
+    return (x.dtype == w.dtype == torch.bfloat16 and x.dim() == w.dim() == 3 and x.device == w.device
+            and 0 < x.shape[1] == w.shape[0] <= 65535 and 0 < x.shape[2] == w.shape[1] and 0 < w.shape[2] <= 1 << 20
+            and x.stride(2) == w.stride(1) == 1 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+            and all(n % 8 == 0 for n in (x.shape[2], w.shape[2], x.stride(0), x.stride(1), w.stride(0), w.stride(2))))
+
+
+def head_product(x, w):
+    """`x [T, H, K]` times `w [H, K, N]` per head, fp32 sums, one rounding -> `[T, H, N]`.  K is innermost in both; the other strides are
+    any whole 16-byte units."""
+    T, H, K = x.shape
+    out = torch.empty((T, H, w.shape[2]), dtype=x.dtype, device=x.device)
+    _check(lib().sglb_head_product(_p(out), x.data_ptr(), x.stride(0), x.stride(1), w.data_ptr(), w.stride(0), w.stride(2), T, H,
+                                   w.shape[2], K, _stream()), "head_product")
     return out
 
 

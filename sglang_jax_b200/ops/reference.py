@@ -314,6 +314,11 @@ def grouped_gemm(x, w, group_sizes):
 
 
 # ----------------------------------------------------------------------------- MLA
+def head_product(x, w):
+    """`x [T, H, K]` times `w [H, K, N]` per head, in fp32."""
+    return torch.einsum("thk,hkn->thn", x.float(), w.float()).to(x.dtype)
+
+
 def mla_paged_attention(q_nope_latent, q_pe, kv_buffer, page_table, req_pool_indices, seq_lens,
                         page_size, scale, kv_lora_rank, cu_q_lens=None, prefix_lens=None, allowed=None, window=0,
                         sink=None):

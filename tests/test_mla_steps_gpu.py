@@ -95,3 +95,53 @@ def test_mla_extend(news, prefixes, page):
     # keys and values (or latent queries and sums) are rounded to bf16 once, 2^-9 of each at most; so is the result
     err = (got.view(T, 4, 96).double() - want).norm() / want.norm()
     assert err < 6e-3, float(err)
+
+
+def _one_rounding(got, x, w):
+    """`got` against `x [T, H, K] . w [H, K, N]`: one rounding to bf16 (eight significant bits: 2^-8 of the value), and fp32 sums of at most 64
+    steps of the tensor core, 2^-22 each of what has been added up.  Two partial sums rounded to bf16 do not pass at K = 512."""
+    want = torch.einsum("thk,hkn->thn", x.double(), w.double())
+    size = torch.einsum("thk,hkn->thn", x.double().abs(), w.double().abs())
+    return ((got.double() - want).abs() <= want.abs() * 2 ** -8 * (1 + 2 ** -8) + size * 2 ** -16 + 1e-30).all()
+
+
+# the sizes of the kernels' rule on a B200: 16-token CTAs up to 1036 of them, tiles of 32 x 64, tiles of 128 x 128
+@pytest.mark.parametrize("T,H,K,N", [(1, 1, 8, 8), (7, 16, 128, 512), (16, 16, 512, 128), (17, 3, 40, 136), (33, 16, 128, 512), (64, 128, 512, 128),
+                                     (65, 128, 512, 128), (129, 16, 200, 520), (260, 16, 128, 512), (1000, 16, 512, 128), (131, 128, 72, 24)])
+def test_head_product(T, H, K, N):
+    torch.manual_seed(T + K)
+    bf = torch.bfloat16
+    wide = torch.randn(T, H, K + 24, device="cuda", dtype=bf)
+    rows = torch.randn(H, N + 8, K, device="cuda", dtype=bf) * K ** -0.5
+    x, w = wide[..., 8:8 + K], rows[:, 8:].transpose(1, 2)           # strides of a wider projection, rows of a taller one
+    from sglang_jax_b200.ops import native
+    assert native.head_product_supported(x, w)
+    got = ops.head_product(x, w)
+    assert got.shape == (T, H, N) and got.is_contiguous() and _one_rounding(got, x, w)
+    assert _one_rounding(ops.head_product(wide[..., 7:7 + K], w), wide[..., 7:7 + K], w)      # not aligned: the general statement
+    assert ops.head_product(x[:0], w).shape == (0, H, N)
+
+
+@pytest.mark.parametrize("T", [1, 7, 96])
+@pytest.mark.parametrize("heads", [16, 128])
+def test_absorbed_products_sum_in_fp32(T, heads, monkeypatch):
+    """The products before and behind latent decode keep fp32 sums whatever the process lets a library do."""
+    from sglang_jax_b200.models.deepseek_v3 import MLAAttention
+    cfg = SimpleNamespace(hidden_size=64, num_attention_heads=heads, qk_nope_head_dim=128, qk_rope_head_dim=64, v_head_dim=128,
+                          kv_lora_rank=512, q_lora_rank=None, rms_norm_eps=1e-6, max_position_embeddings=1024)
+    torch.manual_seed(T)
+    with torch.device("cuda"):
+        m = MLAAttention(cfg, 0, torch.bfloat16)
+    m.kv_b_proj.weight.data.normal_(0, 512 ** -0.5)
+    m.absorb()
+    q = torch.randn(T, heads, 192, device="cuda", dtype=torch.bfloat16)
+    o_lat = torch.randn(T, heads, 512, device="cuda", dtype=torch.bfloat16)
+    monkeypatch.setattr(torch.backends.cuda.matmul, "allow_bf16_reduced_precision_reduction", True)
+
+    def library(*a, **k):
+        raise AssertionError("a library product, whose partial sums that flag lets into bf16")
+
+    monkeypatch.setattr(torch, "bmm", library)
+    up = m.kv_b_proj.weight.view(heads, 256, 512)
+    assert _one_rounding(m._latent_query(q), q[..., :128], up[:, :128])
+    assert _one_rounding(m._value_up(o_lat), o_lat, up[:, 128:].transpose(1, 2))
