@@ -30,11 +30,18 @@ class LinearBase(nn.Module):
         self.bias = _param(out_features, dtype=dtype) if bias else None
         self.lora = None   # set by lora.layers.wrap_linear
         self.qweight = None   # utils.quantization.QuantizedWeight once the layer is quantised
+        self.joint = None     # JointProjection whose allocation holds the weight, if any
 
     def set_quantized(self, qw):
         """Replace the dense weight by quantised storage (the dense tensor is released)."""
         self.qweight = qw
         self.weight = None
+        self.leave_joint()
+
+    def leave_joint(self):
+        """The weight goes elsewhere: so do those that share an allocation with it, which would keep all of it alive."""
+        if self.joint is not None:
+            self.joint.separate()
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if self.qweight is not None:
@@ -149,11 +156,20 @@ class JointProjection:
             row = 0
             for lin, t in zip(linears, w):
                 lin.weight = nn.Parameter(base.narrow(0, row, t.shape[0]), requires_grad=False)
+                lin.joint = self
                 row += t.shape[0]
+
+    def separate(self):
+        """Every weight in an allocation of its own, for good."""
+        for lin in self.linears:
+            lin.joint = None
+            if lin.weight is not None and lin.weight.untyped_storage().nbytes() > lin.weight.numel() * lin.weight.element_size():
+                lin.weight.data = lin.weight.data.clone()
+        self.linears = []
 
     def weight(self) -> torch.Tensor | None:
         """The weights as one matrix, or None."""
-        first = self.linears[0].weight
+        first = self.linears[0].weight if self.linears else None
         if first is None:
             return None
         at, rows, K = first.data_ptr(), 0, first.shape[1]

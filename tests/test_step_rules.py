@@ -22,3 +22,49 @@ def test_router_logits_takes_operands_that_fit(rows, weight, bias, ok):
 def test_router_logits_refuses_what_a_product_refuses():
     with pytest.raises(RuntimeError):
         ops.router_logits(torch.zeros(4, 64, dtype=BF), torch.zeros(8, 32, dtype=BF))
+
+
+# ---- weights of several projections in one allocation
+def _delta_net(width=64):
+    from types import SimpleNamespace
+    from sglang_jax_b200.layers.linear_attention import GatedDeltaNet
+    m = GatedDeltaNet(SimpleNamespace(hidden_size=width, rms_norm_eps=1e-6, linear_num_value_heads=8, linear_num_key_heads=4,
+                                      linear_key_head_dim=16, linear_value_head_dim=16, linear_conv_kernel_dim=4), 0, BF)
+    for p in m.parameters():
+        p.data.normal_()
+    return m
+
+
+def _kept(*linears):
+    """Bytes of the allocations that the layers' weights keep alive beyond their own."""
+    return sum(w.untyped_storage().nbytes() - w.numel() * w.element_size() for w in (lin.weight for lin in linears))
+
+
+def test_a_quantised_projection_releases_its_dense_weight():
+    from sglang_jax_b200.utils.quantization import QuantizedWeight, quantize_tensor
+    m = _delta_net()
+    x = torch.randn(5, 64).to(BF)
+    y, parts = m._joint(x)
+    assert y.shape[1] == sum(p.shape[1] for p in parts) and torch.equal(parts[1], m.in_proj_ba(x)) and torch.equal(parts[0], m.in_proj_qkvz(x))
+    before = m.in_proj_ba.weight.clone()
+    q, s = quantize_tensor(m.in_proj_qkvz.weight.data, torch.int8, "per_channel")
+    m.in_proj_qkvz.set_quantized(QuantizedWeight(q, s, None, None, BF))
+    assert m.in_proj_qkvz.weight is None and _kept(m.in_proj_ba) == 0
+    assert torch.equal(m.in_proj_ba.weight, before) and m._joint(x) is None and m.in_proj_ba(x).shape == (5, 16)
+
+
+def test_a_projection_of_another_type_leaves_the_allocation():
+    from sglang_jax_b200.configs.dtype_config import DtypeConfig, apply_dtype_config
+    m = _delta_net()
+    before = m.in_proj_qkvz.weight.clone()
+    assert list(apply_dtype_config(m, DtypeConfig({"in_proj_ba": "float32"}, torch.bfloat16))) == ["in_proj_ba.weight"]
+    assert _kept(m.in_proj_qkvz, m.in_proj_ba) == 0 and m.in_proj_ba.weight.dtype == torch.float32
+    assert torch.equal(m.in_proj_qkvz.weight, before) and m._joint(torch.zeros(1, 64, dtype=BF)) is None
+
+
+def test_projections_stay_together_where_nothing_changes():
+    from sglang_jax_b200.configs.dtype_config import DtypeConfig, apply_dtype_config
+    m = _delta_net()
+    assert apply_dtype_config(m, DtypeConfig({}, torch.bfloat16)).keys().isdisjoint({"in_proj_qkvz.weight", "in_proj_ba.weight"})
+    m.in_proj_ba.weight_loader(m.in_proj_ba.weight, torch.ones(16, 64))
+    assert m._joint(torch.ones(1, 64, dtype=BF))[1][1].eq(64).all()
