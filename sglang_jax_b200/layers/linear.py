@@ -38,6 +38,11 @@ class LinearBase(nn.Module):
         self.weight = None
         self.leave_joint()
 
+    def plain(self) -> bool:
+        """Whether the layer is `x weight^T` and nothing else: dense, without a bias or an adapter, and nobody watches its calls."""
+        return (self.weight is not None and self.qweight is None and self.lora is None and self.bias is None
+                and not self._forward_hooks and not self._forward_pre_hooks and "forward" not in self.__dict__)
+
     def leave_joint(self):
         """The weight goes elsewhere: so do those that share an allocation with it, which would keep all of it alive."""
         if self.joint is not None:
@@ -144,8 +149,8 @@ class PackedColumnParallelLinear(LinearBase):
 class JointProjection:
     """Several projections of one input as a single product, while each stays a layer of its own: their weights are made
     neighbours in one allocation, so that one product over all of them gives every result as a column range.  `joint(x)` is
-    None where that does not hold (any more): a layer with a bias, quantised or with an adapter, another type for one of them, a
-    weight that was replaced or moved.  Whether it does is read off the weights themselves on every call."""
+    None where that does not hold (any more): a layer that is more than its product (`LinearBase.plain`), another type for one of them,
+    a weight that was replaced or moved.  Whether it does is read off the weights themselves on every call."""
 
     def __init__(self, linears: list[LinearBase]):
         self.linears = linears
@@ -169,14 +174,13 @@ class JointProjection:
 
     def weight(self) -> torch.Tensor | None:
         """The weights as one matrix, or None."""
-        first = self.linears[0].weight if self.linears else None
-        if first is None:
+        if not self.linears or not all(lin.plain() for lin in self.linears):
             return None
+        first = self.linears[0].weight
         at, rows, K = first.data_ptr(), 0, first.shape[1]
         for lin in self.linears:
             w = lin.weight
-            if (w is None or lin.qweight is not None or lin.lora is not None or lin.bias is not None or w.dtype != first.dtype
-                    or w.data_ptr() != at or w.shape[1] != K or not w.is_contiguous()
+            if (w.dtype != first.dtype or w.data_ptr() != at or w.shape[1] != K or not w.is_contiguous()
                     or w.untyped_storage().data_ptr() != first.untyped_storage().data_ptr()):
                 return None
             at += w.numel() * w.element_size()

@@ -373,7 +373,7 @@ class KimiDeltaAttention(_RecurrentMixer):
     @staticmethod
     def _up(lin, part):
         """Second product of a low-rank pair; a plain layer reads the column range of the wider product where it is."""
-        if lin.qweight is None and lin.lora is None and lin.bias is None and lin.weight.dtype == part.dtype:
+        if lin.plain() and lin.weight.dtype == part.dtype:
             return ops.linear_part(part, lin.weight)
         return lin(part.contiguous())
 

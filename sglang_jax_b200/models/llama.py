@@ -34,12 +34,11 @@ class DenseMLP(nn.Module):
 
     def activated(self, x):
         """`act_fn(gate_up_proj(x))`, in one kernel where that is a plain product of prefill size."""
-        up = self.gate_up_proj
-        plain = up.qweight is None and up.lora is None and up.bias is None and type(self.act_fn) is SiluAndMul \
-            and not (up._forward_hooks or up._forward_pre_hooks or self.act_fn._forward_hooks or self.act_fn._forward_pre_hooks)
-        if plain and ops.linear_swiglu_supported(x, up.weight):
+        up, act = self.gate_up_proj, self.act_fn
+        if up.plain() and type(act) is SiluAndMul and not act._forward_hooks and not act._forward_pre_hooks \
+                and ops.linear_swiglu_supported(x, up.weight):
             return ops.linear_swiglu(x, up.weight)
-        return self.act_fn(up(x))
+        return act(up(x))
 
     def forward(self, x):
         return self.down_proj(self.activated(x))

@@ -68,3 +68,16 @@ def test_projections_stay_together_where_nothing_changes():
     assert apply_dtype_config(m, DtypeConfig({}, torch.bfloat16)).keys().isdisjoint({"in_proj_qkvz.weight", "in_proj_ba.weight"})
     m.in_proj_ba.weight_loader(m.in_proj_ba.weight, torch.ones(16, 64))
     assert m._joint(torch.ones(1, 64, dtype=BF))[1][1].eq(64).all()
+
+
+def test_a_watched_projection_is_called():
+    """Hooks of a layer see its call: it is not passed by for a product over several layers."""
+    from sglang_jax_b200.layers.linear_attention import KimiDeltaAttention
+    m, x, seen = _delta_net(), torch.randn(3, 64).to(BF), []
+    for add in ("register_forward_hook", "register_forward_pre_hook"):
+        handle = getattr(m.in_proj_ba, add)(lambda *a: seen.append(add))
+        assert m._joint(x) is None
+        KimiDeltaAttention._up(m.in_proj_ba, x)
+        assert seen.pop() == add and not seen
+        handle.remove()
+        assert m._joint(x) is not None
