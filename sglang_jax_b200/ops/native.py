@@ -380,12 +380,14 @@ def rope_parts(q, k, v, positions, cos_sin, q_norm_w, k_norm_w, eps, kv_buffer, 
 
 def rope_qknorm_kvwrite(qkv, positions, cos_sin, q_norm_w, k_norm_w, eps, num_q_heads, num_kv_heads, head_dim,
                         kv_buffer, out_cache_loc, page_size, is_neox=True, rotary_dim=None, gemma_norm=False):
-    qkv = qkv.contiguous()
+    qkv = qkv.contiguous().flatten(1)                     # (rows by heads are the same rows)
+    if qkv.data_ptr() % 16:
+        qkv = qkv.clone()
     T, qs, ks = qkv.shape[0], num_q_heads * head_dim, num_kv_heads * head_dim
     rd, ld, at = rotary_dim or head_dim, qs + 2 * ks, qkv.data_ptr()
-    if head_dim not in (64, 128, 256) or qkv.shape[1] != ld or at % 16 or positions.dtype != torch.int32 \
-            or (cos_sin is not None and (rd % (16 if is_neox else 2) or rd > head_dim)) \
-            or (kv_buffer is not None and out_cache_loc.dtype != torch.int32) \
+    if head_dim not in (64, 128, 256) or qkv.shape[1] != ld or positions.dtype != torch.int32 \
+            or (cos_sin is not None and (rd % (16 if is_neox else 2) or rd > head_dim or cos_sin.data_ptr() % 16)) \
+            or (kv_buffer is not None and (out_cache_loc.dtype != torch.int32 or kv_buffer.data_ptr() % 16)) \
             or any(w is not None and (w.dtype != torch.bfloat16 or w.data_ptr() % 16) for w in (q_norm_w, k_norm_w)):
         from . import reference
         return reference.rope_qknorm_kvwrite(qkv, positions, cos_sin, q_norm_w, k_norm_w, eps, num_q_heads,

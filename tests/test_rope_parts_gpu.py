@@ -49,3 +49,25 @@ def test_linear_swiglu(T, K, I):
     err = lambda y: ((y.double() - want).norm() / want.norm()).item()
     assert err(ops.linear_swiglu(x, w)) < 2 ** -8                             # one rounding to bf16
     assert err(ops.linear_swiglu(x, w)) <= err(ops.silu_and_mul(ops.linear(x, w)))
+
+
+@pytest.mark.parametrize("form", ["heads", "odd rows", "odd table", "odd cache"])
+def test_rows_as_callers_have_them(form):
+    """Rows by heads, and tensors that begin off a 16-byte boundary: the same results as plain ones."""
+    T, Hq, Hkv, D, P, dev, bf = 37, 3, 1, 64, 16, "cuda", torch.bfloat16
+    torch.manual_seed(5)
+    odd = lambda t: torch.empty(t.numel() + 1, device=dev, dtype=t.dtype)[1:].view_as(t).copy_(t)
+    qkv, pos = torch.randn(T, (Hq + 2 * Hkv) * D, device=dev, dtype=bf), torch.randint(0, 90, (T,), device=dev, dtype=torch.int32)
+    cs, loc = ref.build_cos_sin_cache(D, 90, 1e4, device=dev), torch.randperm(64, device=dev)[:T].int()
+    w = torch.randn(2, D, device=dev, dtype=bf)
+    cache = torch.zeros(4, 2, Hkv, P, D, device=dev, dtype=bf)
+    run = lambda x, table, kv: ops.rope_qknorm_kvwrite(x, pos, table, w[0], w[1], 1e-6, Hq, Hkv, D, kv, loc, P)
+    want = run(qkv, cs, cache)
+    x = {"heads": qkv.view(T, -1, D), "odd rows": odd(qkv)}.get(form, qkv)
+    other = odd(torch.zeros_like(cache)) if form == "odd cache" else torch.zeros_like(cache)
+    got = run(x, odd(cs) if form == "odd table" else cs, other)
+    if form in ("odd table", "odd cache"):               # the general statement: sums in another order, last places of bf16
+        assert (got.float() - want.float()).norm() <= 2e-3 * want.float().norm()
+        assert (other.float() - cache.float()).norm() <= 2e-3 * cache.float().norm()
+    else:
+        assert torch.equal(got, want) and torch.equal(other, cache)
