@@ -89,3 +89,14 @@ def test_layer_equals_its_statements(kind, heads, kv, dim, dtype, weights):
         pool = _pool(m, 5, dtype, 3)
         assert ops.delta_supported(x, pool.conv_state[0], pool.recurrent_state[0], dim, dim, 4) and conv_w.dtype == dtype
         _both(m, x, new, cached, decode, dtype, _tol(dtype))
+
+
+@pytest.mark.parametrize("kind", ["gdn", "kda"])
+def test_decode_with_windows_in_fp32(kind, monkeypatch):
+    """Windows kept in fp32 beside bf16 inputs: the in-place kernels of `csrc/linear_attn.cu`."""
+    m = _layer(kind, 4, 4, 64, BF, 2)
+    calls = []
+    step = native.delta_rule_step
+    monkeypatch.setattr(native, "delta_rule_step", lambda *a, **k: calls.append(1) or step(*a, **k))
+    _both(m, torch.randn(5, 256, device="cuda").to(BF), [1] * 5, [40, 10, 5, 97, 70], True, torch.float32, _tol(BF))
+    assert len(calls) == 1                                 # (the statements do not call it)
