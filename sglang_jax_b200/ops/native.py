@@ -618,13 +618,10 @@ def gemm_fp8(xq, wq, scale_x, scale_w, bias=None, out_dtype=torch.bfloat16):
     return out.view(*xq.shape[:-1], N)
 
 
-def delta_rule_step(q, k, v, g, beta, state_pool, slots, gate_per_channel=False, l2norm=True, rows=None):
+def delta_rule_step(q, k, v, g, beta, state_pool, slots, gate_per_channel=False, l2norm=True):
     """One recurrent step per request, state updated in place.  `q, k [B, Hqk, Dk]`, `v [B, H, Dv]` bf16,
     `g [B, H]` (or `[B, H, Dk]`) and `beta [B, H]` fp32, `state_pool [slots, H, Dk, Dv]` fp32,
-    `slots [B]` int64 -> `o [B, H, Dv]` bf16.  `rows`: the step's inputs are the rows of a projection instead, and the
-    convolution in front of them is part of the step (arguments of `delta_scan`, whose result it returns)."""
-    if rows is not None:
-        return _delta_rows(*rows[0], **rows[1])
+    `slots [B]` int64 -> `o [B, H, Dv]` bf16."""
     B, H, Dv = v.shape
     q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
     g, beta = g.float().contiguous(), beta.float().contiguous()
@@ -1015,21 +1012,14 @@ def latent_extend(q, kv, k_rot, out, plan, dim, v_dim, scale, window=0, sink=Non
 # ---- gated delta rule over ragged batches (csrc/delta_scan.cu)
 def delta_scan(proj, g_off, b_off, a_off, conv_w, a_log, dt_bias, conv_state, state, slots, heads, kv_heads, dim, vdim,
                cu=None, prefix=None, track_len=None, track_slot=None, lens=None, channel_a=None, ba=None, grouped=None):
-    """Read-outs fp32 `[T, heads, vdim]` of the rows of `proj [T, ld]` (columns `q | k | v` first, gate / beta / decay
-    inputs at the given offsets, or those of `ba` if given); `grouped`: the columns of one q / k head and of the value heads that
-    use it, all neighbours, in a row that is `kv_heads` such groups (q, k and v first in each); then beta and decay inputs are
-    grouped as well, a group's betas first.  Windows and states of `slots` are updated in place.  `cu [B + 1]` / `prefix [B]`:
-    ragged step (None: one row per request, all of them continuing); `lens`: its sequence lengths on the host, if known
-    (without them the kernel for single tokens is launched on the chance that there are some).  `channel_a [T, heads * dim]`:
-    one decay per head and key channel from these inputs, `dt_bias [heads * dim]` (`a_off` is not used then)."""
-    args = (proj, g_off, b_off, a_off, conv_w, a_log, dt_bias, conv_state, state, slots, heads, kv_heads, dim, vdim)
-    if cu is None:
-        return delta_rule_step(None, None, None, None, None, state, slots, rows=(args, dict(channel_a=channel_a, ba=ba, grouped=grouped)))
-    return _delta_rows(*args, cu, prefix, track_len, track_slot, lens, channel_a, ba, grouped)
-
-
-def _delta_rows(proj, g_off, b_off, a_off, conv_w, a_log, dt_bias, conv_state, state, slots, heads, kv_heads, dim, vdim,
-                cu=None, prefix=None, track_len=None, track_slot=None, lens=None, channel_a=None, ba=None, grouped=None):
+    """Read-outs fp32 `[T, heads, vdim]` of the rows of `proj [T, ld]` (columns `q | k | v` first, beta and decay inputs at the
+    given offsets, those of `ba` if given; the gate's offset `g_off` is not read).  `grouped`: the columns of one q / k head and
+    of the value heads that use it, all neighbours, in a row that is `kv_heads` such groups (q, k and v first in each); then beta
+    and decay inputs are grouped as well, a group's betas first.  Windows and states of `slots` are updated in place.
+    `cu [B + 1]` / `prefix [B]`: ragged step (None: one row per request, all of them continuing); `lens`: its sequence lengths on
+    the host, if known (without them the kernel for single tokens is launched on the chance that there are some).
+    `channel_a [T, heads * dim]`: one decay per head and key channel from these inputs, `dt_bias [heads * dim]` (`a_off` is not
+    used then)."""
     T, dev, B = proj.shape[0], proj.device, slots.numel()
     singles = 0 if cu is None else (int((lens == 1).sum()) if lens is not None else -1)
     f32 = dict(dtype=torch.float32, device=dev)

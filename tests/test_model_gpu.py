@@ -368,18 +368,18 @@ def test_qwen3_next_decode_with_recurrent_kernels(tmp_path):
     pool = runner.recurrent_pool
     conv0, rec0 = pool.conv_state.clone(), pool.recurrent_state.clone()
     calls = {"n": 0}
-    orig = native.delta_rule_step
+    orig = native.delta_scan
 
     def counted(*a, **k):
         calls["n"] += 1
         return orig(*a, **k)
 
-    native.delta_rule_step = counted
+    native.delta_scan = counted
     try:
         dbatch = _decode_batch(runner, lens, toks)
         d_n, _, _ = runner.forward(dbatch, skip_sample=True)
     finally:
-        native.delta_rule_step = orig
+        native.delta_scan = orig
     assert calls["n"] == 2                                     # the two linear-attention layers
     conv_n, rec_n = pool.conv_state.clone(), pool.recurrent_state.clone()
     pool.conv_state.copy_(conv0)
