@@ -323,7 +323,7 @@ class FusedMoE(nn.Module):
                                                     topk_weights, topk_ids, self.expert_start, self.workspace, add,
                                                     out)
             return moe_native.fused_experts(x, self.w13_weight, self.w2_weight, topk_weights, topk_ids,
-                                            self.expert_start, self.workspace, add, out)
+                                            self.expert_start, self.workspace, add, out, self.num_experts)
         if self.activation in ("clipped_swiglu", "swiglu") and not self.fp8 and ops.use_native(x) and x.shape[1] % 8 == 0:
             from ..ops import moe_native
             ws = self._workspace(topk_ids.numel(), x.device)

@@ -113,12 +113,12 @@ def moe_gather(x, ws: MoeWorkspace, max_rows: int):
     return out
 
 
-def on_pairs(rows: int, K: int, experts: int) -> bool:
-    """Whether a grouped product of `rows` rows runs on pairs of SMs (`csrc/gemm_pair.cu`): its maps want whole blocks of 64 lanes.  Up
-    to 256 rows the other kernel shares the bytes of all experts out evenly over all SMs, which is good while most of few experts are
+def on_pairs(rows: int, K: int, experts: int, expected: int | None = None) -> bool:
+    """Whether a grouped product of `rows` rows at most (`expected` of them, where others may be other ranks') runs on pairs of SMs
+    (`csrc/gemm_pair.cu`): its maps want whole blocks of 64 lanes.  Up to 256 rows the other kernel shares the bytes of all experts out evenly over all SMs, which is good while most of few experts are
     chosen.  Both products of 768 x 2048, pairs against that, 64 experts: 37 / 66 us at 8 rows, 96 / 88 at 56, 125 / 118 at 128,
     135 / 137 at 256; 128 experts: 117 / 134 at 64 rows, 206 / 232 at 256."""
-    return K % 64 == 0 and (rows > 256 or experts >= 128 or 2 * rows <= experts)
+    return K % 64 == 0 and (rows > 256 or experts >= 128 or 2 * (rows if expected is None else expected) <= experts)
 
 
 def pair_tile(rows: int, experts: int) -> int:
@@ -129,6 +129,15 @@ def pair_tile(rows: int, experts: int) -> int:
     mean = max(rows // max(experts, 1), 1)
     n = -(-mean // 256)
     return min(256, -(-mean * 5 // (4 * n * 32)) * 32)
+
+
+def expert_tile(pairs: int, hidden: int, inner: int, local: int, experts: int) -> int:
+    """Rows of a token tile for both products of `local` of all `experts` on pairs of SMs, 0 where they run elsewhere.  `pairs` (token,
+    choice) pairs of the step are spread over all experts, those of other ranks too: this rank's rows are its share of them."""
+    rows = -(-pairs * local // max(experts, 1))
+    if on_pairs(pairs, hidden, local, rows) and on_pairs(pairs, inner, local, rows):
+        return pair_tile(rows, local)
+    return 0
 
 
 def grouped_gemm_pair(x_sorted, w, ws: MoeWorkspace, rows: int, gated: bool = False):
@@ -248,22 +257,22 @@ def moe_combine(y_sorted, topk_weights, ws: MoeWorkspace, T: int, add=None, out=
 
 
 def fused_experts(x, w13, w2, topk_weights, topk_ids, expert_start: int = 0, ws: MoeWorkspace | None = None,
-                  add=None, out=None):
+                  add=None, out=None, experts: int | None = None):
     """Routed-expert FFN with the native kernels: align -> gather -> grouped GEMM (gate|up) -> SiLU*mul ->
-    grouped GEMM (down) -> weighted combine.  `w13 [E_local, 2I, H]`, `w2 [E_local, H, I]`."""
+    grouped GEMM (down) -> weighted combine.  `w13 [E_local, 2I, H]`, `w2 [E_local, H, I]`; `experts`: of all ranks (None: these)."""
     T, H = x.shape
     k = topk_ids.shape[1]
     E_local = w13.shape[0]
     pairs = T * k
     if ws is None or ws.max_pairs < pairs:
         ws = MoeWorkspace(pairs, E_local, x.device)
-    if on_pairs(pairs, H, E_local) and on_pairs(pairs, w2.shape[2], E_local):
-        moe_align(topk_ids, expert_start, E_local, ws, tile_rows=pair_tile(pairs, E_local))
-        a = grouped_gemm_pair(moe_gather(x, ws, pairs), w13, ws, pairs, gated=True)
+    tile = expert_tile(pairs, H, w2.shape[2], E_local, experts or E_local)
+    if tile:
+        moe_align(topk_ids, expert_start, E_local, ws, tile_rows=tile)
+        y = grouped_gemm_pair(grouped_gemm_pair(moe_gather(x, ws, pairs), w13, ws, pairs, gated=True), w2, ws, pairs)
     else:
         moe_align(topk_ids, expert_start, E_local, ws)
-        a = native.silu_and_mul(grouped_gemm(moe_gather(x, ws, pairs), w13, ws, pairs))
-    y = grouped_gemm(a, w2, ws, pairs)
+        y = grouped_gemm(native.silu_and_mul(grouped_gemm(moe_gather(x, ws, pairs), w13, ws, pairs)), w2, ws, pairs)
     return moe_combine(y, topk_weights, ws, T, add=add, out=out)
 
 

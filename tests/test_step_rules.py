@@ -81,3 +81,14 @@ def test_a_watched_projection_is_called():
         assert seen.pop() == add and not seen
         handle.remove()
         assert m._joint(x) is not None
+
+
+# ---- expert products under expert parallelism
+@pytest.mark.parametrize("pairs,local,experts,tile", [
+    (8192, 32, 256, 64), (8192, 256, 256, 64), (8192, 32, 32, 256),       # 32 rows an expert on one of eight ranks are 32 on a single one
+    (16384, 16, 128, 160), (16384, 128, 128, 160),
+    (64, 64, 512, 32), (64, 64, 64, 0),                                   # 8 rows for 64 experts: most of them idle
+    (260, 8, 64, 32), (260, 8, 8, 64)])
+def test_expert_tiles_follow_this_ranks_rows(pairs, local, experts, tile):
+    assert moe_native.expert_tile(pairs, 2048, 768, local, experts) == tile
+    assert moe_native.expert_tile(pairs, 2040, 768, local, experts) == moe_native.expert_tile(pairs, 2048, 760, local, experts) == 0
