@@ -2,6 +2,7 @@
 
 from __future__ import annotations
 
+from functools import cached_property
 from typing import NamedTuple
 
 import numpy as np
@@ -35,9 +36,7 @@ class ExtendPlan:
         long = np.nonzero(n >= MIN_TILE_TOKENS)[0] if tiles else np.empty(0, np.int64)
         dev = fb.positions.device
         self.long = len(long)
-        # every token as a query of its own: its sequence's row, and the tokens up to and including itself
-        self.token_rows = torch.repeat_interleave(fb.req_pool_indices, fb.extend_seq_lens.long(), output_size=fb.num_tokens)
-        self.token_lens = fb.positions + 1
+        self._tokens = fb.req_pool_indices, fb.extend_seq_lens, fb.num_tokens, fb.positions
         self.short_tokens = None
         if self.long:
             self._prefix, self._end, self._contexts = pre[long], (pre + n)[long], {}
@@ -54,6 +53,15 @@ class ExtendPlan:
                 if len(short):
                     self.short_tokens = torch.from_numpy(short).to(dev)
 
+    # every token as a query of its own: its sequence's row, and the tokens up to and including itself
+    @cached_property
+    def token_rows(self) -> torch.Tensor:
+        rows, n, total, _ = self._tokens
+        return torch.repeat_interleave(rows, n.long(), output_size=total)
+
+    @cached_property
+    def token_lens(self) -> torch.Tensor:
+        return self._tokens[3] + 1
 
     def context(self, window: int = 0) -> Context:
         """What the long sequences see under a window (0: everything), from a multiple of `KEY_TILE` on."""

@@ -158,22 +158,19 @@ class MLAAttention(nn.Module):
                 ops.latent_extend(q[:, h0:h1], kv, pe, o[:, h0:h1], plan, self.nope, self.v_dim, self.scaling)
             if plan.short_tokens is None:
                 return o
-        rows, lens = self._token_view(fb)
         t = slice(None) if plan.short_tokens is None else plan.short_tokens
         qs = q[t]
-        o[t] = self._value_up(ops.mla_tokens(self._latent_query(qs), qs[..., self.nope:], buf, fb, self.scaling, rows[t], lens[t]))
+        o[t] = self._value_up(ops.mla_tokens(self._latent_query(qs), qs[..., self.nope:], buf, fb, self.scaling, plan.token_rows[t],
+                                             self._token_lens(fb)[t]))
         return o
 
     @staticmethod
-    def _token_view(fb):
-        """Page-table row of every new token and the tokens it sees (by its place in the sequence, whatever its position id)."""
-        if "mla_token_view" not in fb.extras:
-            n = fb.extend_seq_lens.long()
-            first = fb.extend_prefix_lens - fb.cu_q_lens[:-1]
-            seq = torch.repeat_interleave(torch.arange(len(n), device=n.device), n, output_size=fb.num_tokens)
-            lens = first[seq] + torch.arange(1, fb.num_tokens + 1, dtype=torch.int32, device=n.device)
-            fb.extras["mla_token_view"] = fb.req_pool_indices[seq], lens
-        return fb.extras["mla_token_view"]
+    def _token_lens(fb):
+        """The tokens that every new one sees: by its place in the sequence, whatever its position id."""
+        if "mla_token_lens" not in fb.extras:
+            first = torch.repeat_interleave(fb.extend_prefix_lens - fb.cu_q_lens[:-1], fb.extend_seq_lens.long(), output_size=fb.num_tokens)
+            fb.extras["mla_token_lens"] = first + torch.arange(1, fb.num_tokens + 1, dtype=torch.int32, device=first.device)
+        return fb.extras["mla_token_lens"]
 
 
 class DeepseekMoE(nn.Module):
