@@ -145,3 +145,38 @@ def test_absorbed_products_sum_in_fp32(T, heads, monkeypatch):
     up = m.kv_b_proj.weight.view(heads, 256, 512)
     assert _one_rounding(m._latent_query(q), q[..., :128], up[:, :128])
     assert _one_rounding(m._value_up(o_lat), o_lat, up[:, 128:].transpose(1, 2))
+
+
+@pytest.mark.parametrize("group", [1, 3])
+def test_mla_extend_in_groups_of_heads(group, monkeypatch):
+    """Where the expanded keys and values of all heads are too much at a time, the heads go in groups (the last one shorter): each is
+    computed by itself, so the bits are the same."""
+    from sglang_jax_b200.models.deepseek_v3 import MLAAttention
+    torch.manual_seed(group)
+    bf, page, n, pre = torch.bfloat16, 16, [40, 5, 300], [70, 20, 0]
+    cfg = SimpleNamespace(hidden_size=256, num_attention_heads=4, qk_nope_head_dim=64, qk_rope_head_dim=32, v_head_dim=96,
+                          kv_lora_rank=128, q_lora_rank=None, rms_norm_eps=1e-6, max_position_embeddings=1024)
+    with torch.device("cuda"):
+        m = MLAAttention(cfg, 0, bf)
+    for p in m.parameters():
+        p.data.normal_(0, 0.06)
+    m.absorb()
+    t = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    total = [a + b for a, b in zip(n, pre)]
+    table = (torch.randperm(3 * 20, device="cuda") + 1).int().view(3, 20)
+    cache = torch.randn(61, page, 160, device="cuda", dtype=bf)
+    q = torch.randn(sum(n), 4, 96, device="cuda", dtype=bf)
+    pos = t([i for a, b in zip(pre, n) for i in range(a, a + b)])
+
+    def run():
+        fb = SimpleNamespace(positions=pos, page_table=table, req_pool_indices=t([0, 1, 2]), seq_lens=t(total), page_size=page,
+                             extend_seq_lens_cpu=np.asarray(n), extend_prefix_lens_cpu=np.asarray(pre), extend_seq_lens=t(n),
+                             extend_prefix_lens=t(pre), cu_q_lens=t([0, 40, 45, 345]), num_tokens=sum(n), max_seq_len=max(total), extras={})
+        return m._extend(q, cache, fb)
+
+    want, groups = run(), []
+    long = sum(a for a, b in zip(total, n) if b >= 32)     # tokens of which keys and values are expanded
+    monkeypatch.setattr(m, "EXPAND_BYTES", group * long * (64 + 96) * 2)
+    extend = ops.latent_extend
+    monkeypatch.setattr(ops, "latent_extend", lambda q, *a: groups.append(q.shape[1]) or extend(q, *a))
+    assert torch.equal(run(), want) and groups == ([1] * 4 if group == 1 else [3, 1])
