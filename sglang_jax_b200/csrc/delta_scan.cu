@@ -1046,12 +1046,12 @@ int launch_prep(const DeltaParams& p, cudaStream_t s) {
   auto blocks = [&](int run) {
     return dim3(static_cast<unsigned>(((static_cast<long long>(p.T) + run - 1) / run * units + 3) / 4));
   };
-  // long runs reuse the window and the kernel; short steps want the warps.  Eight rows a warp from 16 warps an SM on (1024 rows of 32
-  // units: 78 us a row at a time, 38 so), sixteen from 32 of those on
-  const long long rows = static_cast<long long>(p.T) * units;
-  if (p.cu != nullptr && rows >= 16 * 148 * 32)
+  // long runs reuse the window and the kernel; short steps want the warps.  Eight rows a warp from 16 such warps an SM on (1024 rows of 32
+  // units: 78 us a row at a time, 38 so), sixteen from 32 on
+  const long long rows = static_cast<long long>(p.T) * units, sms = sm_count();
+  if (p.cu != nullptr && rows >= 16 * sms * 32)
     launch_pdl(delta_prep_kernel<T, NPL, TAPS, 16>, blocks(16), dim3(128), 0, s, p);
-  else if (p.cu != nullptr && rows >= 8 * 148 * 16)
+  else if (p.cu != nullptr && rows >= 8 * sms * 16)
     launch_pdl(delta_prep_kernel<T, NPL, TAPS, 8>, blocks(8), dim3(128), 0, s, p);
   else
     launch_pdl(delta_prep_kernel<T, NPL, TAPS, 1>, blocks(1), dim3(128), 0, s, p);
