@@ -1,5 +1,6 @@
 // Decode-step kernels of the linear-attention token mixers (Gated DeltaNet of Qwen3-Next / Qwen3.5,
-// Kimi Delta Attention): the per-request recurrent state lives in a slot pool and is updated in place.
+// Kimi Delta Attention) for convolution windows that are not of the inputs' type (fp32 beside bf16; where they are,
+// delta_scan.cu runs): the per-request recurrent state lives in a slot pool and is updated in place.
 //
 //   delta_rule_step   S <- diag-or-scalar decay * S;  S <- S + k (beta (v - S^T k))^T;  o = S^T q
 //                     one CTA per (request, value head); thread j owns column j of the [Dk, Dv] state and

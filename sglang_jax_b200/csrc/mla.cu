@@ -461,7 +461,7 @@ int sglb_mla_num_splits(int B, int groups, int max_seq_len) {
 // Absorbed-MLA decode.  `kv_buffer` is the latent cache [num_pages, page_size, row_elems] (bf16, rows of
 // kv_lora_rank + rope_dim lanes and padding, row_elems a multiple of 8); `q_lat` [B, H, kv_lora_rank], `q_pe` addressed
 // by strides; `out` [B, H, kv_lora_rank].  With `num_splits > 1` the partial buffers `part_o [B, H, splits, R]` and
-// `part_lse [B, H, splits]` (fp32) are required.  `exact`: attention weights are not rounded to bf16.  `window` (0: none):
+// `part_lse [B, H, splits]` (fp32) are required.  `exact`: attention weights enter as two bf16 terms.  `window` (0: none):
 // tokens a query sees, its own included; `sink` [H] or null.
 int sglb_mla_decode(const void* q_lat, const void* q_pe, long long pe_token_stride, int pe_head_stride, void* out,
                     const void* kv_buffer, long long num_pages, int row_elems, const int* page_table, int max_pages,

@@ -130,9 +130,13 @@ class MLAAttention(nn.Module):
     def _tiled(self, q, q_pe, buf, fb, allowed) -> bool:
         """Whether the sequences of an extend step can go through the prefill kernel (long ones: keys and values of what they see
         are expanded from the latents by one GEMM) and the decode kernel (short ones, token by token).  Absorbed, a (query, key)
-        pair costs R + rot + R products instead of dim + rot + v: 1088 against 320 at 512 + 64 latent lanes; from 32 new tokens on
-        the expansion costs less than that.  Four layers of 16 heads, 3000 new tokens: 21.8 ms a step with fp32 products over the
-        latents, 3.4 ms in this way, and closer to 64-bit arithmetic (0.0026 of the result's norm, not 0.0027)."""
+        pair costs R + rot + R products instead of dim + rot + v: 1088 against 320 at 512 + 64 latent lanes; the expansion costs
+        512 x 256 for every key.  In products alone that is even at 171 new tokens, but the tiles run on tcgen05 and the tokens on
+        mma.sync.  A layer in us, tiles / tokens: 8 sequences behind 512 tokens, 16 heads 45 / 40 at 8 new tokens each, 45 / 89 at 31, 46 / 121
+        at 64; behind 4096 231 / 118, 230 / 336, 234 / 612; 128 heads 1742 / 616, 1771 / 2132, 1786 / 4280.  One sequence of 16 heads gives
+        the tiles 16 CTAs: 107 / 66 at 32 new tokens behind 4096 and 675 / 341 behind 30000, 107 / 118 and 675 / 649 at 64.  Four layers of 16
+        heads, 3000 new tokens: 21.8 ms a step with fp32 products over the latents, 3.4 ms in this way; error against 64-bit arithmetic
+        (16 heads, 3000 tokens behind 512) 0.0042 of the result's norm instead of 0.0045."""
         n = fb.extend_seq_lens_cpu
         return (allowed is None and n is not None and int(n.sum()) == q.shape[0] == fb.num_tokens
                 and ops.latent_extend_supported(q, self.nope, self.rope_dim, self.v_dim, self.kv_lora)

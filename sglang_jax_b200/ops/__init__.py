@@ -424,8 +424,8 @@ def mla_tokens_supported(q_pe, cache, heads: int, rank: int, page_size: int) -> 
 
 
 def mla_tokens(q_latent, q_pe, cache, fb, scale, rows, lens):
-    """Absorbed attention of query tokens on their own, unrounded weights: query n sees the first `lens[n]` tokens of page-table
-    row `rows[n]`."""
+    """Absorbed attention of query tokens on their own, weights as sums of two bf16 numbers: query n sees the first `lens[n]` tokens
+    of page-table row `rows[n]`."""
     return _native().mla_decode(q_latent, q_pe, cache, fb.page_table, rows, lens, fb.page_size, scale, fb.max_seq_len, exact=True)
 
 

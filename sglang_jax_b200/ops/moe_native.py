@@ -115,9 +115,12 @@ def moe_gather(x, ws: MoeWorkspace, max_rows: int):
 
 def on_pairs(rows: int, K: int, experts: int, expected: int | None = None) -> bool:
     """Whether a grouped product of `rows` rows at most (`expected` of them, where others may be other ranks') runs on pairs of SMs
-    (`csrc/gemm_pair.cu`): its maps want whole blocks of 64 lanes.  Up to 256 rows the other kernel shares the bytes of all experts out evenly over all SMs, which is good while most of few experts are
-    chosen.  Both products of 768 x 2048, pairs against that, 64 experts: 37 / 66 us at 8 rows, 96 / 88 at 56, 125 / 118 at 128,
-    135 / 137 at 256; 128 experts: 117 / 134 at 64 rows, 206 / 232 at 256."""
+    (`csrc/gemm_pair.cu`): its maps want whole blocks of 64 lanes.  Up to 256 rows the other kernel shares the bytes of all experts
+    out evenly over all SMs, which is good while most of few experts are chosen.  Both products of 768 x 2048, pairs against that, 64
+    experts: 37 / 66 us at 8 rows, 96 / 88 at 56, 125 / 118 at 128, 135 / 137 at 256; 128 experts: 117 / 134 at 64 rows, 206 / 232 at 256.
+    Whole layers at other sizes, rows spread evenly: 16 experts of 1408 x 4096 98 / 92 at 32 rows, 103 / 140 at 256, 48 of them 149 / 165 and
+    263 / 343; 80 of 768 x 2048 81 / 96 at 64 rows, 128 / 158 at 256, 112 of them 93 / 116 and 162 / 216.  So from some 48 experts on and for
+    wider ones the line is on the safe side: what it sends to the other kernel there would be faster in pairs."""
     return K % 64 == 0 and (rows > 256 or experts >= 128 or 2 * (rows if expected is None else expected) <= experts)
 
 

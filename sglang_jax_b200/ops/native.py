@@ -666,7 +666,7 @@ def mla_decode(q_latent, q_pe, kv_buffer, page_table, req_pool_indices, seq_lens
                num_splits=None, exact=False, window=0, sink=None):
     """Absorbed-MLA decode: `q_latent [B, H, R]`, `q_pe [B, H, rotary lanes]` (any strides, unit innermost), latent
     cache `[pages, P, row]` with `row >= R + rotary lanes` -> latent output `[B, H, R]` (the caller applies W_UV).
-    `exact`: the attention weights enter the value product unrounded.  `window` (0: none): tokens a query sees, its own
+    `exact`: the attention weights enter the value product as sums of two bf16 numbers (16 bits), else rounded to one.  `window` (0: none): tokens a query sees, its own
     included; `sink` fp32 `[H]`: joins the softmax's denominator."""
     B, H, R = q_latent.shape
     q_latent = q_latent.contiguous()
