@@ -28,30 +28,30 @@ def _layer(kind, heads, kv, dim, dtype, seed):
     return m
 
 
-def _batch(new, cached, decode, pool):
+def _batch(new, cached, decode, pool, tracks):
     i32 = lambda v: torch.tensor(np.asarray(v, np.int32), device="cuda")
     new, cached = np.asarray(new), np.asarray(cached)
     return SimpleNamespace(forward_mode=SimpleNamespace(is_decode=lambda: decode), cu_q_lens=i32(np.concatenate([[0], np.cumsum(new)])),
                            extend_prefix_lens=i32(cached), extend_prefix_lens_cpu=cached, extend_seq_lens_cpu=new, batch_size=len(new),
                            req_pool_indices=i32(np.arange(len(new))[::-1].copy()), positions=i32(np.zeros(int(new.sum()))),
-                           extras={"recurrent_pool": pool})
+                           extras={"recurrent_pool": pool, "recurrent_tracks": tracks})
 
 
 def _pool(m, B, conv_dtype, seed):
     torch.manual_seed(seed)
     heads, dim = (m.nh, m.hd) if hasattr(m, "nh") else (m.nv, m.dk)
-    return SimpleNamespace(conv_state=torch.randn(1, B + 1, m.conv_dim, 3, device="cuda").to(conv_dtype),
-                           recurrent_state=torch.randn(1, B + 1, heads, dim, dim, device="cuda") * 0.1)
+    return SimpleNamespace(conv_state=torch.randn(1, B + 3, m.conv_dim, 3, device="cuda").to(conv_dtype),
+                           recurrent_state=torch.randn(1, B + 3, heads, dim, dim, device="cuda") * 0.1)
 
 
-def _both(m, x, new, cached, decode, conv_dtype, tol):
+def _both(m, x, new, cached, decode, conv_dtype, tol, tracks=None):
     """The layer as it runs and by its statements, from the same caches."""
     got = []
     for reference in (False, True):
         pool = _pool(m, len(new), conv_dtype, 3)
         ops.set_force_reference(reference)
         try:
-            y = m(x, _batch(new, cached, decode, pool))
+            y = m(x, _batch(new, cached, decode, pool, tracks))
         finally:
             ops.set_force_reference(False)
         got.append((y, pool.conv_state, pool.recurrent_state))
@@ -88,7 +88,8 @@ def test_layer_equals_its_statements(kind, heads, kv, dim, dtype, weights):
         x = torch.randn(sum(new), 256, device="cuda").to(dtype)
         pool = _pool(m, 5, dtype, 3)
         assert ops.delta_supported(x, pool.conv_state[0], pool.recurrent_state[0], dim, dim, 4) and conv_w.dtype == dtype
-        _both(m, x, new, cached, decode, dtype, _tol(dtype))
+        # checkpoints inside and at the end of a sequence, in slots of their own
+        _both(m, x, new, cached, decode, dtype, _tol(dtype), None if decode else {0: (32, 6), 4: (70, 7)})
 
 
 @pytest.mark.parametrize("kind", ["gdn", "kda"])
