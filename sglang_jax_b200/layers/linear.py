@@ -30,13 +30,13 @@ class LinearBase(nn.Module):
         self.bias = _param(out_features, dtype=dtype) if bias else None
         self.lora = None   # set by lora.layers.wrap_linear
         self.qweight = None   # utils.quantization.QuantizedWeight once the layer is quantised
-        self.joint = None     # JointProjection whose allocation holds the weight, if any
+        self.joint: list[nn.Parameter] = []     # weights in one allocation, this one's among them (`JointProjection`)
 
     def set_quantized(self, qw):
         """Replace the dense weight by quantised storage (the dense tensor is released)."""
+        self.leave_joint()
         self.qweight = qw
         self.weight = None
-        self.leave_joint()
 
     def plain(self) -> bool:
         """Whether the layer is `x weight^T` and nothing else: dense, without a bias or an adapter, and nobody watches its calls."""
@@ -45,8 +45,10 @@ class LinearBase(nn.Module):
 
     def leave_joint(self):
         """The weight goes elsewhere: so do those that share an allocation with it, which would keep all of it alive."""
-        if self.joint is not None:
-            self.joint.separate()
+        for w in self.joint:
+            if w is not self.weight:
+                w.data = w.data.clone()
+        self.joint.clear()
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if self.qweight is not None:
@@ -161,20 +163,14 @@ class JointProjection:
             row = 0
             for lin, t in zip(linears, w):
                 lin.weight = nn.Parameter(base.narrow(0, row, t.shape[0]), requires_grad=False)
-                lin.joint = self
                 row += t.shape[0]
-
-    def separate(self):
-        """Every weight in an allocation of its own, for good."""
-        for lin in self.linears:
-            lin.joint = None
-            if lin.weight is not None and lin.weight.untyped_storage().nbytes() > lin.weight.numel() * lin.weight.element_size():
-                lin.weight.data = lin.weight.data.clone()
-        self.linears = []
+            together = [lin.weight for lin in linears]
+            for lin in linears:
+                lin.joint = together
 
     def weight(self) -> torch.Tensor | None:
         """The weights as one matrix, or None."""
-        if not self.linears or not all(lin.plain() for lin in self.linears):
+        if not all(lin.plain() for lin in self.linears):
             return None
         first = self.linears[0].weight
         at, rows, K = first.data_ptr(), 0, first.shape[1]

@@ -62,6 +62,27 @@ def test_a_projection_of_another_type_leaves_the_allocation():
     assert torch.equal(m.in_proj_qkvz.weight, before) and m._joint(torch.zeros(1, 64, dtype=BF)) is None
 
 
+def test_a_layer_goes_when_its_last_reference_does():
+    import gc
+    import weakref
+    gc.disable()
+    try:
+        m = _delta_net()
+        watch = weakref.ref(m.in_proj_qkvz)
+        del m
+        assert watch() is None                   # no cycle through the shared allocation waits for a collection
+    finally:
+        gc.enable()
+
+
+def test_copies_share_nothing_with_the_original():
+    import copy
+    m = _delta_net()
+    c = copy.deepcopy(m)
+    c.in_proj_qkvz.leave_joint()
+    assert m._joint(torch.zeros(1, 64, dtype=BF)) is not None and torch.equal(c.in_proj_ba.weight, m.in_proj_ba.weight)
+
+
 def test_projections_stay_together_where_nothing_changes():
     from sglang_jax_b200.configs.dtype_config import DtypeConfig, apply_dtype_config
     m = _delta_net()
