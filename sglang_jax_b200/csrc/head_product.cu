@@ -4,12 +4,13 @@
 // Partial sums never leave fp32, whatever the sizes (a library may add up the pieces of a split product in the type of its result).
 // Operands are read where they lie: heads of a token and heads of the weights by strides.
 //
-//   head_product_few_kernel    decode: 16 tokens x 16 columns of a head a CTA, four warps share K; bound by latency
+//   head_product_few_kernel    decode: 16 tokens x 16 columns of a head a CTA, its warps share K; bound by latency
 //   head_product_tile_kernel   more tokens or heads: tiles through a ring in shared memory (cp.async), one tile a CTA; a tile has two to
 //                              eight stages, so that it is bound by their latency in a short pipeline, then by L2
 //
-// fp32 products on the CUDA cores took 17 and 20 us at 96 tokens of 16 heads (128 -> 512 and 512 -> 128 lanes), these 3.2 and 3.5; a batched
-// library product in bf16, whose sums may be split and added up in bf16, 2.9 and 3.1.
+// 16 heads, 128 -> 512 and 512 -> 128 lanes, weights from DRAM as in a step: 7 tokens 2.5 and 3.0 us, 96 tokens 3.5 and 4.9; a batched library
+// product in bf16, whose sums may be split and added up in bf16, 3.5 and 3.8, 3.8 and 4.1; fp32 products on the CUDA cores (weights in L2) 17
+// and 20 at 96 tokens.
 #include "common.cuh"
 #include "mma_sync.cuh"
 
@@ -34,13 +35,14 @@ struct HeadProductParams {
   }
 };
 
-constexpr int kFewWarps = 4, kFewCols = 16, kFewRuns = 4;
+constexpr int kFewCols = 16;
 
-// Operands come straight from L2, 16 bytes a load: inside a run of 32 lanes of K both have the same permutation, and a warp has four runs
-// in flight.
-__global__ void __launch_bounds__(32 * kFewWarps)
+// Operands come straight from memory, 16 bytes a load: inside a run of 32 lanes of K both have the same permutation.  A warp has RUNS runs
+// in flight, all of K in one go for what is usual (4 warps x 1 run of 128 lanes, 8 x 2 of 512).
+template <int WARPS, int RUNS>
+__global__ void __launch_bounds__(32 * WARPS)
 head_product_few_kernel(const HeadProductParams p) {
-  __shared__ float part[kFewWarps][16][kFewCols];
+  __shared__ float part[WARPS][16][kFewCols];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   const int t0 = blockIdx.x * 16, n0 = blockIdx.y * kFewCols, h = blockIdx.z;
   pdl_wait();
@@ -51,11 +53,11 @@ head_product_few_kernel(const HeadProductParams p) {
     wb[i] = p.w_row(n0 + 8 * i + g, h) + 8 * t4;
   }
   float c[2][4] = {};
-  for (int k0 = 32 * warp; k0 < p.K; k0 += 32 * kFewWarps * kFewRuns) {
-    uint4 a[kFewRuns][2], b[kFewRuns][2];
+  for (int k0 = 32 * warp; k0 < p.K; k0 += 32 * WARPS * RUNS) {
+    uint4 a[RUNS][2], b[RUNS][2];
 #pragma unroll
-    for (int r = 0; r < kFewRuns; ++r) {
-      const int k = k0 + 32 * kFewWarps * r;
+    for (int r = 0; r < RUNS; ++r) {
+      const int k = k0 + 32 * WARPS * r;
       const bool in = k + 8 * t4 < p.K;                       // (K is whole groups of 8 lanes; zeros add nothing)
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
@@ -64,7 +66,7 @@ head_product_few_kernel(const HeadProductParams p) {
       }
     }
 #pragma unroll
-    for (int r = 0; r < kFewRuns; ++r) {
+    for (int r = 0; r < RUNS; ++r) {
       const uint32_t lo[4] = {a[r][0].x, a[r][1].x, a[r][0].y, a[r][1].y}, hi[4] = {a[r][0].z, a[r][1].z, a[r][0].w, a[r][1].w};
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
@@ -78,10 +80,11 @@ head_product_few_kernel(const HeadProductParams p) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) part[warp][g + 8 * (i >> 1)][8 * n + 2 * t4 + (i & 1)] = c[n][i];
   __syncthreads();
+  if (threadIdx.x >= 16 * kFewCols / 2) return;
   const int t = threadIdx.x / (kFewCols / 2), n = threadIdx.x % (kFewCols / 2) * 2;
   float v0 = 0.f, v1 = 0.f;
 #pragma unroll
-  for (int q = 0; q < kFewWarps; ++q) {
+  for (int q = 0; q < WARPS; ++q) {
     v0 += part[q][t][n];
     v1 += part[q][t][n + 1];
   }
@@ -95,10 +98,8 @@ __device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool in) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
 }
 
-constexpr int kTileStages = 3;
-
-// BM tokens x BN columns of one head, 64 lanes of K a stage; WM x WN warps.
-template <int BM, int BN, int WM, int WN>
+// BM tokens x BN columns of one head, 64 lanes of K a stage, STAGES of the ring; WM x WN warps.
+template <int BM, int BN, int WM, int WN, int STAGES>
 __global__ void __launch_bounds__(32 * WM * WN)
 head_product_tile_kernel(const HeadProductParams p) {
   constexpr int kThreads = 32 * WM * WN, kStage = (BM + BN) * 128, MT = BM / WM / 16, NT = BN / WN / 16;
@@ -110,7 +111,7 @@ head_product_tile_kernel(const HeadProductParams p) {
   pdl_wait();
   auto load = [&](int kb) {
     if (kb < blocks) {
-      const uint32_t st = base + kb % kTileStages * kStage;
+      const uint32_t st = base + kb % STAGES * kStage;
 #pragma unroll
       for (int i = threadIdx.x; i < (BM + BN) * 8; i += kThreads) {
         const int row = i >> 3, k = kb * 64 + (i & 7) * 8;
@@ -122,13 +123,13 @@ head_product_tile_kernel(const HeadProductParams p) {
     asm volatile("cp.async.commit_group;" ::: "memory");      // (an empty one past the end: the count below stays right)
   };
 #pragma unroll
-  for (int s = 0; s < kTileStages - 1; ++s) load(s);
+  for (int s = 0; s < STAGES - 1; ++s) load(s);
   float c[MT][NT][2][4] = {};
   for (int kb = 0; kb < blocks; ++kb) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(kTileStages - 2) : "memory");
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
     __syncthreads();                                          // the stage has landed; the one before it is read
-    load(kb + kTileStages - 1);
-    const uint32_t sa = base + kb % kTileStages * kStage, sb = sa + BM * 128;
+    load(kb + STAGES - 1);
+    const uint32_t sa = base + kb % STAGES * kStage, sb = sa + BM * 128;
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
       uint32_t a[MT][4], b[NT][4];
@@ -159,13 +160,20 @@ head_product_tile_kernel(const HeadProductParams p) {
       }
 }
 
-template <int BM, int BN, int WM, int WN>
+template <int WARPS, int RUNS>
+cudaError_t launch_few(const HeadProductParams& p, cudaStream_t s) {
+  static_assert(32 * WARPS >= 16 * kFewCols / 2, "a thread for every pair of results");
+  return launch_pdl(head_product_few_kernel<WARPS, RUNS>, dim3((p.T + 15) / 16, (p.N + kFewCols - 1) / kFewCols, p.H), dim3(32 * WARPS), 0, s,
+                    p);
+}
+
+template <int BM, int BN, int WM, int WN, int STAGES>
 cudaError_t launch_tile(const HeadProductParams& p, cudaStream_t s) {
-  constexpr int smem = kTileStages * (BM + BN) * 128;
+  constexpr int smem = STAGES * (BM + BN) * 128;
   static const cudaError_t configured =
-      cudaFuncSetAttribute(head_product_tile_kernel<BM, BN, WM, WN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      cudaFuncSetAttribute(head_product_tile_kernel<BM, BN, WM, WN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (configured != cudaSuccess) return configured;
-  return launch_pdl(head_product_tile_kernel<BM, BN, WM, WN>, dim3((p.T + BM - 1) / BM, (p.N + BN - 1) / BN, p.H), dim3(32 * WM * WN), smem,
+  return launch_pdl(head_product_tile_kernel<BM, BN, WM, WN, STAGES>, dim3((p.T + BM - 1) / BM, (p.N + BN - 1) / BN, p.H), dim3(32 * WM * WN), smem,
                     s, p);
 }
 
@@ -187,15 +195,17 @@ int sglb_head_product(void* out, const void* x, long long x_ts, int x_hs, const 
   const HeadProductParams p{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(out),
                             x_ts, w_hs, x_hs, w_ld, T, H, N, K};
   auto ctas = [&](int m, int n) { return static_cast<long long>((T + m - 1) / m) * ((N + n - 1) / n) * H; };
-  // By CTAs, for 128 -> 512 lanes and 512 -> 128 lanes.  Up to seven a SM the small ones, which share K: 16 heads, 7 tokens 2.1 and
-  // 2.5 us against 2.1 and 4.1 in tiles of 32 x 64, 96 tokens (768 CTAs) 3.5 against 4.3; twice as many (128 heads, 17 tokens) 6.4
-  // against 5.2.  Large tiles where more than half of their rows are tokens and most SMs get one: 16 heads, 256 tokens 4.4 against 5.9 us
-  // (the other product, 32 tiles, 9.8 against 5.3), 1000 tokens 12.9 and 10.1 against 18.3 and 13.8, 128 heads 83 and 58 against 133 and 90.
-  if (ctas(16, kFewCols) <= 7ll * sm_count())
-    return static_cast<int>(launch_pdl(head_product_few_kernel, dim3((T + 15) / 16, (N + kFewCols - 1) / kFewCols, H),
-                                       dim3(32 * kFewWarps), 0, s, p));
-  if (T > 64 && 8 * ctas(128, 128) >= 6ll * sm_count()) return static_cast<int>(launch_tile<128, 128, 4, 2>(p, s));
-  return static_cast<int>(launch_tile<32, 64, 1, 4>(p, s));
+  // (us for weights from DRAM, H heads x T tokens, 128 -> 512 lanes; then 512 -> 128)
+  // The small CTAs up to about 900 threads an SM: 16 x 7 2.5 against 2.8 in tiles, 16 x 32 2.8 / 3.0, 16 x 64 4.0 / 3.2; 16 x 64 3.5 / 4.8,
+  // 16 x 96 5.2 / 4.9, 128 x 7 6.3 / 5.9.  K up to 128 in four warps: 16 x 7 2.5, in eight 2.6; 512 in eight: 3.0, in four 4.4.
+  // Large tiles where more than half of their rows are tokens and most SMs get one: 128 x 96 12.6 against 14.7, 16 x 256 4.7 / 6.4, 16 x 128
+  // (64 tiles) 4.4 / 3.9; 128 x 128 10.9 / 14.7, 16 x 256 (32 tiles) 10.2 / 5.8.
+  const long long few = ctas(16, kFewCols), sms = sm_count();
+  if (K <= 128 && few <= 7 * sms) return static_cast<int>(launch_few<4, 1>(p, s));
+  if (K > 128 && 2 * few <= 7 * sms) return static_cast<int>(launch_few<8, 2>(p, s));
+  if (T > 64 && 8 * ctas(128, 128) >= 6 * sms) return static_cast<int>(launch_tile<128, 128, 4, 2, 3>(p, s));
+  // the ring as deep as helps: 512 lanes 4.9 with five stages, 5.5 with three; 128 lanes (two stages) 3.5 with three, 3.5 with five
+  return static_cast<int>(K > 192 ? launch_tile<32, 64, 1, 4, 5>(p, s) : launch_tile<32, 64, 1, 4, 3>(p, s));
 }
 
 }  // extern "C"

@@ -105,9 +105,11 @@ def _one_rounding(got, x, w):
     return ((got.double() - want).abs() <= want.abs() * 2 ** -8 * (1 + 2 ** -8) + size * 2 ** -16 + 1e-30).all()
 
 
-# the sizes of the kernels' rule on a B200: 16-token CTAs up to 1036 of them, tiles of 32 x 64, tiles of 128 x 128
-@pytest.mark.parametrize("T,H,K,N", [(1, 1, 8, 8), (7, 16, 128, 512), (16, 16, 512, 128), (17, 3, 40, 136), (33, 16, 128, 512), (64, 128, 512, 128),
-                                     (65, 128, 512, 128), (129, 16, 200, 520), (260, 16, 128, 512), (1000, 16, 512, 128), (131, 128, 72, 24)])
+# the kernels' rule on a B200: CTAs of 16 tokens (four warps, K up to 128: up to 1036 of them; eight: 518), tiles of 32 x 64 with a ring of three
+# stages (K up to 192) and of five, tiles of 128 x 128
+@pytest.mark.parametrize("T,H,K,N", [(1, 1, 8, 8), (7, 16, 128, 512), (16, 16, 512, 128), (17, 3, 40, 136), (65, 16, 520, 72), (33, 16, 128, 512),
+                                     (64, 128, 512, 128), (65, 128, 512, 128), (129, 16, 200, 520), (40, 128, 192, 136), (260, 16, 128, 512),
+                                     (1000, 16, 512, 128), (131, 128, 72, 24)])
 def test_head_product(T, H, K, N):
     torch.manual_seed(T + K)
     bf = torch.bfloat16
