@@ -238,18 +238,34 @@ struct RopeParams {
   int page_size;
 };
 
-// One CTA per token (and share of its heads where tokens are few): D / 8 lanes hold a head, 16 bytes each, lane u of the first half of the
-// rotary part turns with lane u + rd / 16.  A thread keeps its cosines, sines and norm weights for all heads that it takes.  Bound by
-// memory: 8192 tokens of 64 + 2 x 8 heads 230 us with 2-byte accesses and a position's row read again for every head, now 135.
+// D / 8 lanes hold a head, 16 bytes each; lane u of the first half of the rotary part turns with lane u + rd / 16.  A CTA takes a token (or a
+// share of its heads where tokens are few), its threads as many heads at a time as divide them well; where one pass holds the heads of several
+// tokens it takes `tokens` of them.  A thread keeps its cosines, sines and norm weights for all heads that it takes.  Bound by memory in prefill, by
+// latency in decode.  With 2-byte accesses and a position's row read again for every head / with one token a CTA of 256 threads whatever its
+// heads / now, us: 8192 tokens of 64 + 2 x 8 normed heads 173 / 105 / 103, 16 + 2 x 4 of them half rotated 46 / 52 / 40, 8 + 2 of 64 lanes 14 / 23 /
+// 9.6, 1 + 2 6.8 / 24 / 6.7; 16 tokens of 8 + 2 2.0 / 2.3 / 1.9, of 40 + 2 x 8 2.4 / 2.4 / 2.0.
 constexpr int kRopeThreads = 256;
 
 template <int D>
 __global__ void __launch_bounds__(kRopeThreads)
-rope_qknorm_kvwrite_kernel(const RopeParams p) {
-  constexpr int L = D / 8, kSlots = kRopeThreads / L;
-  const int t = blockIdx.x, u = threadIdx.x % L, lane = threadIdx.x & 31;
+rope_qknorm_kvwrite_kernel(const RopeParams p, int T, int tokens) {
+  constexpr int L = D / 8;
+  const int u = threadIdx.x % L, lane = threadIdx.x & 31, slot = threadIdx.x / L, slots = blockDim.x / L;
   const int heads = p.Hq + 2 * p.Hkv, half = p.rd / 16;          // vectors in a half
+  const int place = tokens > 1 ? slot / heads : 0, t_own = blockIdx.x * tokens + place;
+  const bool live = place < tokens && t_own < T;
+  const int t = live ? t_own : 0;
+  int h = tokens > 1 ? slot - place * heads : blockIdx.y * slots + slot;
+  const int step = gridDim.y * slots, passes = tokens > 1 ? 1 : (heads - static_cast<int>(blockIdx.y) * slots + step - 1) / step;
   pdl_wait();
+  auto load = [&](int head) {
+    if (!live || head >= heads) return make_uint4(0, 0, 0, 0);
+    const __nv_bfloat16* src = head < p.Hq ? p.q + t * p.q_ts + static_cast<long long>(head) * p.q_hs
+                               : head < p.Hq + p.Hkv ? p.k + t * p.k_ts + static_cast<long long>(head - p.Hq) * D
+                                                     : p.v + t * p.v_ts + static_cast<long long>(head - p.Hq - p.Hkv) * D;
+    return reinterpret_cast<const uint4*>(src)[u];
+  };
+  uint4 raw = load(h);                         // (on its way while the position's row is looked up)
   const bool first = u < half, turns = p.cos_sin != nullptr && u < 2 * half;
   const int partner = lane - u + (first ? u + half : u - half);
   float c[8], sn[8];
@@ -261,35 +277,26 @@ rope_qknorm_kvwrite_kernel(const RopeParams p) {
       c[e] = a.x, c[e + 1] = a.y, c[e + 2] = a.z, c[e + 3] = a.w;
       sn[e] = b.x, sn[e + 1] = b.y, sn[e + 2] = b.z, sn[e + 3] = b.w;
     }
-    if (first) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) sn[e] = -sn[e];
-    }
   }
   uint4 wq = make_uint4(0, 0, 0, 0), wk = wq;
   if (p.q_w != nullptr) wq = reinterpret_cast<const uint4*>(p.q_w)[u];
   if (p.k_w != nullptr) wk = reinterpret_cast<const uint4*>(p.k_w)[u];
   long long slot_at = -1;
   if (p.kv != nullptr) {
-    const int slot = p.loc[t];
-    const int page = slot / p.page_size, off = slot - page * p.page_size;
-    if (slot >= 0) slot_at = (static_cast<long long>(page) * 2 * p.Hkv * p.page_size + off) * D;
+    const int at = p.loc[t];
+    const int page = at / p.page_size, off = at - page * p.page_size;
+    if (at >= 0) slot_at = (static_cast<long long>(page) * 2 * p.Hkv * p.page_size + off) * D;
 #ifdef SGLB_BOUNDS_CHECK
-    if (g_dbg_kv_pages > 0 && (slot < 0 || page >= g_dbg_kv_pages)) {
-      if (threadIdx.x == 0) report(g_dbg_status, kOutOfBounds, t, slot);
+    if (g_dbg_kv_pages > 0 && (at < 0 || page >= g_dbg_kv_pages)) {
+      if (u == 0 && h == 0) report(g_dbg_status, kOutOfBounds, t, at);
       slot_at = -1;
     }
 #endif
   }
   // (all lanes of a warp stay in the loop together: they exchange values)
-  for (int h0 = blockIdx.y * kSlots; h0 < heads; h0 += gridDim.y * kSlots) {
-    const int h = h0 + threadIdx.x / L;
-    const bool is_q = h < p.Hq, is_k = !is_q && h < p.Hq + p.Hkv, in = h < heads;
-    const int hk = is_k ? h - p.Hq : h - p.Hq - p.Hkv;
-    const __nv_bfloat16* src = is_q ? p.q + t * p.q_ts + static_cast<long long>(h) * p.q_hs
-                                    : (is_k ? p.k + t * p.k_ts : p.v + t * p.v_ts) + static_cast<long long>(hk) * D;
-    uint4 raw = make_uint4(0, 0, 0, 0);
-    if (in) raw = reinterpret_cast<const uint4*>(src)[u];
+  for (int i = 0; i < passes; ++i, h += step) {
+    if (i > 0) raw = load(h);
+    const bool is_q = h < p.Hq, is_k = !is_q && h < p.Hq + p.Hkv, in = live && h < heads;
     const bool norm = is_q ? p.q_w != nullptr : is_k && p.k_w != nullptr;
     if (p.q_w != nullptr || p.k_w != nullptr) {
       float v[8], w[8], ss = 0.f;
@@ -312,7 +319,7 @@ rope_qknorm_kvwrite_kernel(const RopeParams p) {
         unpack8(raw, v);
         unpack8(other, o);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = v[e] * c[e] + o[e] * sn[e];
+        for (int e = 0; e < 8; ++e) v[e] = v[e] * c[e] + o[e] * (first ? -sn[e] : sn[e]);
         raw = pack8(v);
       }
     }
@@ -320,7 +327,7 @@ rope_qknorm_kvwrite_kernel(const RopeParams p) {
     if (is_q) {
       reinterpret_cast<uint4*>(p.q_out + (static_cast<long long>(t) * p.Hq + h) * D)[u] = raw;
     } else if (slot_at >= 0) {
-      const long long head = static_cast<long long>(is_k ? hk : hk + p.Hkv) * p.page_size * D;
+      const long long head = static_cast<long long>(h - p.Hq) * p.page_size * D;      // (values behind the keys)
       reinterpret_cast<uint4*>(p.kv + slot_at + head)[u] = raw;
     }
   }
@@ -399,11 +406,20 @@ cudaError_t launch_rope(const RopeParams& p, long long T, bool pairs, cudaStream
     const long long blocks = (T * heads * 32 + 127) / 128;
     return launch_pdl(rope_pairs_kernel<D>, dim3(blocks), dim3(128), 0, s, p, T);
   }
-  // few tokens: a token's heads go to several CTAs, until there are a few for every SM
-  const int shares = (heads + kRopeThreads / (D / 8) - 1) / (kRopeThreads / (D / 8));
-  const long long want = (4ll * sm_count() + T - 1) / T;
-  return launch_pdl(rope_qknorm_kvwrite_kernel<D>, dim3(static_cast<unsigned>(T), static_cast<unsigned>(want < shares ? want : shares)),
-                    dim3(kRopeThreads), 0, s, p);
+  constexpr int kMost = kRopeThreads / (D / 8), kWarp = 32 / (D / 8);            // heads of a CTA at a time; of a warp
+  const long long want = 4ll * sm_count();                                       // CTAs to have at least, if there is work for them
+  auto threads = [](int h) { return dim3((h + kWarp - 1) / kWarp * 32); };
+  if (heads <= kMost) {
+    const long long most = kMost / heads, some = T / want;
+    const int tokens = static_cast<int>(some < 1 ? 1 : some < most ? some : most);
+    return launch_pdl(rope_qknorm_kvwrite_kernel<D>, dim3(static_cast<unsigned>((T + tokens - 1) / tokens)), threads(tokens * heads), 0, s, p,
+                      static_cast<int>(T), tokens);
+  }
+  // few tokens: a token's passes go to several CTAs
+  const int passes = (heads + kMost - 1) / kMost;
+  const long long shares = (want + T - 1) / T;
+  return launch_pdl(rope_qknorm_kvwrite_kernel<D>, dim3(static_cast<unsigned>(T), static_cast<unsigned>(shares < passes ? shares : passes)),
+                    threads((heads + passes - 1) / passes), 0, s, p, static_cast<int>(T), 1);
 }
 
 // page_table[rows[i], pos[i]] = ids[i]

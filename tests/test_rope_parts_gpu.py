@@ -71,3 +71,28 @@ def test_rows_as_callers_have_them(form):
         assert (other.float() - cache.float()).norm() <= 2e-3 * cache.float().norm()
     else:
         assert torch.equal(got, want) and torch.equal(other, cache)
+
+
+# heads that fill a CTA's pass, several tokens to a CTA (some of its lanes idle, the last CTA with fewer tokens), passes of uneven shares; tokens
+# from where on the CTAs are enough for several each (592 on a B200)
+@pytest.mark.parametrize("Hq,Hkv,D", [(1, 1, 128), (8, 1, 64), (3, 1, 256), (14, 1, 128), (16, 4, 128), (16, 2, 256), (7, 5, 64), (30, 1, 64)])
+@pytest.mark.parametrize("T", [1, 591, 1187, 2961])
+def test_rope_spreads_heads_over_threads(Hq, Hkv, D, T):
+    torch.manual_seed(T + Hq)
+    dev, bf, P = "cuda", torch.bfloat16, 16
+    qkv = torch.randn(T, (Hq + 2 * Hkv) * D, device=dev, dtype=bf)
+    pos = torch.randint(0, 500, (T,), device=dev, dtype=torch.int32)
+    cs = ref.build_cos_sin_cache(D // 2, 500, 1e4, device=dev)
+    w = torch.randn(2, D, device=dev, dtype=bf) * 0.2 + 1.0
+    loc = torch.randperm(T + 40, device=dev)[:T].int()
+    loc[::7] = -1                                        # tokens whose keys and values go nowhere
+    cache = torch.zeros((T + 40) // P + 1, 2, Hkv, P, D, device=dev, dtype=bf)
+    got = ops.rope_qknorm_kvwrite(qkv, pos, cs, w[0], w[1], 1e-6, Hq, Hkv, D, cache, loc, P, True, D // 2)
+    kept, want_kv = loc >= 0, torch.zeros_like(cache)
+    want = ref.rope_qknorm_kvwrite(qkv, pos, cs, w[0], w[1], 1e-6, Hq, Hkv, D, None, loc, P, True, D // 2)
+    ref.rope_qknorm_kvwrite(qkv[kept], pos[kept], cs, w[0], w[1], 1e-6, Hq, Hkv, D, want_kv, loc[kept], P, True, D // 2)
+    # sums in another order: a norm's rounding to bf16 may fall the other way, and a rotation adds two such values and rounds again
+    for a, b in ((got, want), (cache, want_kv)):
+        assert (a.float() - b.float()).abs().max() <= 2 ** -6 * max(b.float().abs().max().item(), 1.0)
+        assert (a.float() - b.float()).norm() <= 2e-3 * b.float().norm()
+    assert torch.equal(cache[:, 1], want_kv[:, 1])
