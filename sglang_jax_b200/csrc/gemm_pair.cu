@@ -382,7 +382,35 @@ int pick_tile(int T, int cols, int blocks) {
   return best;
 }
 
+// Microseconds of a dense product, fitted to 886 sizes (257 to 8192 tokens, 8 to 28672 columns, K 64 to 14336; operands in L2 where they
+// fit).  Here: a start that grows with the tile, blocks of K as in pick_tile, and for each further wave the longer of its products and
+// its epilogue (3.9 us for 256 x 256).  On single SMs (gemm_sm100.cu, mode 0): 0.3 us a block of K whatever the tile, a little more once
+// operands no longer stay in L2, a further wave of 128 x 256 tiles 2.9 us for its epilogue.  The choice by them is more than 5% off the
+// better one at 8 of these sizes, 8.5% at most.
+float pair_us(int T, int cols, int blocks) {
+  const int bt = pick_tile(T, cols, blocks), pairs = std::max(sm_count() / 2, 1);
+  const float share = bt / 256.f, slice = std::max(0.34f * share, 0.14f + 0.11f * share);
+  const long long waves = (static_cast<long long>((T + bt - 1) / bt) * cols + pairs - 1) / pairs;
+  return 5.1f + 2.6f * share + slice * blocks + (waves - 1) * std::max(3.85f * share, 2.1f * share + 0.95f * slice * blocks);
+}
+float single_us(int T, int N, int blocks, int bn) {
+  const long long waves = (static_cast<long long>((T + 127) / 128) * ((N + bn - 1) / bn) + sm_count() - 1) / sm_count();
+  if (bn == 256) return 5.9f + 0.329f * blocks + 0.04f * std::max(blocks - 64, 0) + (waves - 1) * std::max(2.9f, 1.3f + 0.378f * blocks);
+  return 4.9f + 0.302f * blocks + (waves - 1) * std::max(1.45f, 0.65f + 0.302f * blocks);
+}
+
 }  // namespace
+
+// Pairs are the better choice for most sizes (2500 x 2048 -> 2048 35 -> 27 us, 8192 x 4096 -> 10240 528 -> 441), but not where K is short,
+// so that a tile is mostly epilogue (8192 x 64 -> 28672: 141 us on single SMs, 189 here; 4096 x 512 -> 4096 20.8 / 24.3), nor where the tiles
+// of single SMs fill one wave as well and theirs are half as large (1000 x 2048 -> 4096: 17.4 / 19.0; 300 x 1536 -> 10240: 14.5 / 16.5).
+// Fewer than 64 columns for many tokens, which read the tokens and do little else, are outside the fit: 8192 x 4096 -> 8 23.8 / 32.4, but
+// 4096 x 7168 -> 8 47.1 / 37.3.
+bool gemm_pair_pays(int T, int N, int K, int single_bn) {
+  if (K % BK) return false;
+  if (N < 64 && T > 1024 && K <= 4096) return false;
+  return pair_us(T, (N + 2 * kRows - 1) / (2 * kRows), K / BK) <= single_us(T, N, K / BK, single_bn);
+}
 
 int gemm_pair(const void* x, long long ldx, const void* w, const void* bias, void* out, int T, int N, int K, bool gated,
               const GemmGroups* groups, int bt, cudaStream_t stream) {

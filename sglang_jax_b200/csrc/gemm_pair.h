@@ -10,6 +10,9 @@ struct GemmGroups {
   int count;
 };
 
+// Whether a dense product of more than 256 tokens is faster here than in tiles of 128 x `single_bn` on single SMs.
+bool gemm_pair_pays(int T, int N, int K, int single_bn);
+
 int gemm_pair(const void* x, long long ldx, const void* w, const void* bias, void* out, int T, int N, int K, bool gated,
               const GemmGroups* groups, int bt, cudaStream_t stream);
 

@@ -10,7 +10,7 @@
 //
 // Two operand assignments share the kernel:
 //   MODE 0 ("tokens on M")   A = x tile (128 tokens), B = w tile (BN outputs).  Prefill of what gemm_pair.cu does not take:
-//          fp8, products fused with a collective, K that is no multiple of 64.
+//          fp8, products fused with a collective, K that is no multiple of 64 or short, sizes whose tiles fill one wave here.
 //   MODE 1 ("weights on M")  A = w tile (128 outputs), B = x (all tokens, BN >= M).  Decode:
 //          the 128-row MMA dimension is filled with weight rows, so a batch of 1..256 tokens
 //          wastes no tensor-core rows, weights are streamed exactly once, and K is split over
@@ -1113,10 +1113,12 @@ int sglb_gemm_bf16_impl(const void* x, const void* w, const void* bias, void* ou
   }();
   int mode = force_mode >= 0 ? force_mode : (M <= 256 ? decode_mode : 0);
   if (mode == 1 && M > 256) mode = 0;
-  // Prefill sizes run on pairs of SMs (figures there).  Its maps split K into blocks of 64, so other K stay with the tiles below, as do
-  // fp8 operands and products fused with a collective; up to 256 tokens the weights are the only traffic that counts, and every SM
-  // streams an equal share of them (128 tokens, 5120 -> 51200: 109 us here, 112 us in pairs).
-  if (force_mode < 0 && M > 256 && K % BK == 0 && !fp8 && fused == nullptr && rs_world == 0)
+  // tokens on M: 256 columns a tile where that fills the SMs or divides N
+  const int wide_bn = (N >= 256 && (static_cast<long long>((M + 127) / 128) * ((N + 255) / 256) >= sm_count() || N % 256 == 0)) ? 256 : 128;
+  // Prefill sizes run on pairs of SMs where that is faster (figures there).  Its maps split K into blocks of 64, so other K stay with the
+  // tiles below, as do fp8 operands and products fused with a collective; up to 256 tokens the weights are the only traffic that counts,
+  // and every SM streams an equal share of them (128 tokens, 5120 -> 51200: 109 us here, 112 us in pairs).
+  if (force_mode < 0 && M > 256 && !fp8 && fused == nullptr && rs_world == 0 && gemm_pair_pays(M, N, K, wide_bn))
     return gemm_pair(x, ldx, w, bias, out, M, N, K, false, nullptr, 0, stream);
 
   Params p{};
@@ -1174,8 +1176,7 @@ int sglb_gemm_bf16_impl(const void* x, const void* w, const void* bias, void* ou
   CUtensorMap ta, tb;
   cudaError_t err;
   if (mode == 0) {
-    const int bn = (N >= 256 && (static_cast<long long>((M + 127) / 128) * ((N + 255) / 256) >= sms || N % 256 == 0))
-                       ? 256 : 128;
+    const int bn = wide_bn;
     p.tiles_a = (M + BM - 1) / BM;
     p.tiles_b = (N + bn - 1) / bn;
     if (!encode_tmap_2d(&ta, x, K, M, static_cast<uint64_t>(ldx) * eb, bke, BM, eb)) return -100;

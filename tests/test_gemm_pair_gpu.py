@@ -52,3 +52,18 @@ def test_linear_takes_either_kernel(M, N, K):
     close(got, x.float() @ w.float().t(), K)
     assert (got != general).float().mean() < 0.01
     native.check_status()
+
+
+# a side of every line of the rule: short K, tiles that fill one wave of single SMs, few columns for many tokens
+@pytest.mark.parametrize("M,N,K", [(257, 264, 64), (300, 136, 192), (1000, 4096, 192), (2048, 4096, 512), (300, 10240, 1536), (1025, 56, 256),
+                                   (1024, 56, 2048), (1025, 64, 2048), (2500, 1000, 2048)])
+def test_products_of_either_choice(M, N, K):
+    x, w = operands(M, N, K)
+    bias = w[:, 0].contiguous()
+    want = x.float() @ w.float().t()
+    close(native.linear(x, w), want, K)
+    close(native.linear(x, w, bias), want + bias.float(), K)
+    wide = torch.full((M, K + 72), float("nan"), device="cuda", dtype=torch.bfloat16)
+    wide[:, 8:K + 8] = x
+    assert torch.equal(native.linear_part(wide[:, 8:K + 8], w), native.linear(x, w))
+    native.check_status()
